@@ -41,6 +41,62 @@ struct DevParams {
 };
 
 // ---------------------------------------------------------------------------
+// IEEE quotients and square roots without a branch
+// ---------------------------------------------------------------------------
+
+// a / b for a divisor b known in advance, with y = RN(1/b) precomputed (an IEEE
+// division): Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990)
+// -- if y is 1/b correctly rounded and q is within one ulp of a/b, then
+// r = a - b q is a double (one exact FMA) and RN(q + r y) = RN(a/b). Here
+// q = RN(a y) is within one ulp, so the result equals the IEEE quotient a / b
+// bit for bit (finite a/b in the normal range), in three operations.
+//
+// With y from rcp_cubic(b) instead of the rounded reciprocal, q is still within
+// an ulp or so and r still exact, and what is rounded last, q + r y, differs
+// from a/b by r times y's error: at most 2^-104 of it. So the result is RN(a/b)
+// unless a/b lies within 2^-104 of a rounding midpoint (about one random
+// operand pair in 2^51).
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+    const double q = a * y;
+    const double r = fma(-b, q, a);
+    return fma(r, y, q);
+}
+
+// 1/b within an ulp for b in the normal range whose reciprocal is normal: the
+// hardware estimate x0 (about 2^-20: it sees the upper 32 bits of b) and one
+// third-order step, 1/b = x0 / (1 - e) = x0 (1 + e + e^2 + O(e^3)) with
+// e = 1 - b x0, leaving about 2^-60 before the last rounding. One operation
+// less than two Newton steps. Infinite b gives NaN.
+__device__ __forceinline__ double rcp_cubic(double b) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(b));
+    const double e = fma(-b, x, 1.0);
+    return fma(x, fma(e, e, e), x);
+}
+
+// sqrt(b) for b in [2^-900, 2^900]: the estimate y0 of 1/sqrt b (about 2^-20),
+// one third-order step y = y0 (1 + e/2 + 3 e^2/8), e = 1 - b y0^2, and the
+// final correction s + (b - s^2) y / 2 with the residual exact (one FMA), which
+// leaves 2^-104 before the last rounding: RN(sqrt b) as in div_rcp's note
+// (Markstein 1990). No branch.
+__device__ __forceinline__ double sqrt_cubic(double b) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+    const double e = fma(-(b * y0), y0, 1.0);
+    const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);
+    const double s = b * y;
+    return fma(fma(-s, s, b), 0.5 * y, s);
+}
+
+// x in [2^-900, 2^900): the range in which rcp_cubic, div_rcp and sqrt_cubic
+// neither overflow nor lose a residual to underflow (sign or NaN: false).
+__device__ __forceinline__ bool mid_range(double x) {
+    return (unsigned)(__double2hiint(x) - ((1023 - 900) << 20)) < (1800u << 20);
+}
+__device__ __forceinline__ bool finite_hi(double x) {
+    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+// ---------------------------------------------------------------------------
 // Thermodynamics (field_structures.h:94-105, 405-451)
 // ---------------------------------------------------------------------------
 
@@ -153,6 +209,123 @@ __device__ __forceinline__ void split_lf(R rho, R u, R v, R w, R E, R p, R c, R 
     Fm[2] = R(0.5) * (F3 - a_max * rho * v);
     Fm[3] = R(0.5) * (F4 - a_max * rho * w);
     Fm[4] = R(0.5) * (F5 - a_max * E);
+}
+
+// Split fluxes of one cell raw = (rho, u, v, w, p) as primitiveToConserved and
+// the split of the reference give them (IEEE divisions and square roots).
+template <int FVS, int N1, int N2, int N3>
+__device__ __forceinline__ void split_ieee(double gamma, double eps, const double* raw, double* Fp,
+                                           double* Fm) {
+    double rr = raw[0];
+    if (rr <= 0.0) rr = 1e-12;
+    double E, c;
+    p2c_Ec(rr, raw[1], raw[2], raw[3], raw[4], gamma, E, c);
+    if constexpr (FVS == FV_SW)
+        split_sw<double, N1, N2, N3>(rr, raw[1], raw[2], raw[3], E, raw[4], c, gamma, eps, Fp, Fm);
+    else
+        split_lf<double, N1, N2, N3>(rr, raw[1], raw[2], raw[3], E, raw[4], c, Fp, Fm);
+}
+
+template <int FVS, int N1, int N2, int N3>
+__device__ __noinline__ void split_ieee_cold(double gamma, double eps, const double* raw, double* Fp,
+                                             double* Fm) {
+    split_ieee<FVS, N1, N2, N3>(gamma, eps, raw, Fp, Fm);
+}
+
+// FP64 form of the split: the values of split_ieee, operation for operation,
+// with the quotients and roots from the branch-free forms above (p/((gamma-1)
+// rho) and the two quotients by rho from two reciprocals, rho/(2 gamma) from the
+// constant's), the products with the zero components of the normal left out
+// (they add a zero) and 0.5 (l +- |l|) as the selection it is. States outside
+// the ranges those need take split_ieee: density, pressure or sound speed extreme or not
+// a number, energy not finite. y2g = RN(1 / (2 gamma)).
+template <int FVS, int N1, int N2, int N3>
+__device__ __forceinline__ void split_exact(const DevParams& P, double y2g, const double* raw,
+                                            double Fp[5], double Fm[5]) {
+    static_assert(N1 + N2 + N3 == 1, "axis-aligned face normal");
+    const double gamma = P.gamma, eps = P.sw_eps;
+    double rho = raw[0];
+    if (rho <= 0.0) rho = 1e-12;
+    const double u = raw[1], v = raw[2], w = raw[3], p = raw[4];
+    const double g1r = (gamma - 1.0) * rho;
+    const double yr = rcp_cubic(rho);
+    const double c2 = div_rcp(gamma * p, rho, yr);
+    const double kinetic = 0.5 * (u * u + v * v + w * w);
+    const double E = rho * (div_rcp(p, g1r, rcp_cubic(g1r)) + kinetic);
+    const double c = sqrt_cubic(c2);
+    const double un = N1 ? u : (N2 ? v : w);
+    bool ok = mid_range(rho) && mid_range(p) && mid_range(c2) && finite_hi(E);
+    if constexpr (FVS == FV_SW) {
+        const double l1 = un - c, l2 = un, l3 = un + c;
+        double l1p, l1m, l2p, l2m, l3p, l3m;
+        if (eps > 0.0) {
+            const double e2 = eps * eps;
+            const double b1 = l1 * l1 + e2, b2 = l2 * l2 + e2, b3 = l3 * l3 + e2;
+            const double a1 = sqrt_cubic(b1), a2 = sqrt_cubic(b2), a3 = sqrt_cubic(b3);
+            ok = ok && mid_range(b1) && mid_range(b2) && mid_range(b3);
+            l1p = 0.5 * (l1 + a1); l1m = 0.5 * (l1 - a1);
+            l2p = 0.5 * (l2 + a2); l2m = 0.5 * (l2 - a2);
+            l3p = 0.5 * (l3 + a3); l3m = 0.5 * (l3 - a3);
+        } else {
+            const bool s1 = __double2hiint(l1) < 0, s2 = __double2hiint(l2) < 0, s3 = __double2hiint(l3) < 0;
+            l1p = s1 ? 0.0 : l1; l1m = s1 ? l1 : 0.0;
+            l2p = s2 ? 0.0 : l2; l2m = s2 ? l2 : 0.0;
+            l3p = s3 ? 0.0 : l3; l3m = s3 ? l3 : 0.0;
+        }
+        const double S1p = l1p + l3p, S1m = l1m + l3m, S2p = l3p - l1p, S2m = l3m - l1m;
+        const double H = div_rcp(E + p, rho, yr);
+        const double ga1 = div_rcp(rho, 2.0 * gamma, y2g), ga2 = 2.0 * (gamma - 1.0);
+        const double gp = ga2 * l2p, gm = ga2 * l2m;
+        const double cp = S2p * c, cm = S2m * c;
+        const double vel[3] = {u, v, w};
+        Fp[0] = ga1 * (S1p + gp);
+        Fm[0] = ga1 * (S1m + gm);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const bool normal = d == 0 ? N1 : (d == 1 ? N2 : N3);
+            const double bp = S1p * vel[d] + gp * vel[d], bm = S1m * vel[d] + gm * vel[d];
+            Fp[1 + d] = ga1 * (normal ? bp + cp : bp);
+            Fm[1 + d] = ga1 * (normal ? bm + cm : bm);
+        }
+        Fp[4] = ga1 * (S1p * H + gp * kinetic + S2p * un * c);
+        Fm[4] = ga1 * (S1m * H + gm * kinetic + S2m * un * c);
+        ok = ok && finite_hi(H);
+    } else {
+        const double a_max = fabs(un) + c;
+        const double F1 = rho * un;
+        const double F2 = N1 ? rho * u * un + p : rho * u * un;
+        const double F3 = N2 ? rho * v * un + p : rho * v * un;
+        const double F4 = N3 ? rho * w * un + p : rho * w * un;
+        const double F5 = (E + p) * un;
+        const double ar = a_max * rho, aE = a_max * E;
+        const double au = ar * u, av = ar * v, aw = ar * w;
+        Fp[0] = 0.5 * (F1 + ar); Fm[0] = 0.5 * (F1 - ar);
+        Fp[1] = 0.5 * (F2 + au); Fm[1] = 0.5 * (F2 - au);
+        Fp[2] = 0.5 * (F3 + av); Fm[2] = 0.5 * (F3 - av);
+        Fp[3] = 0.5 * (F4 + aw); Fm[3] = 0.5 * (F4 - aw);
+        Fp[4] = 0.5 * (F5 + aE); Fm[4] = 0.5 * (F5 - aE);
+    }
+    if (!ok) {
+        double r5[5] = {raw[0], u, v, w, p}, P5[5], M5[5];
+        split_ieee_cold<FVS, N1, N2, N3>(gamma, eps, r5, P5, M5);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            Fp[q] = P5[q];
+            Fm[q] = M5[q];
+        }
+    }
+}
+
+// The split of the FP64 sweeps. Linear schemes are bound by memory latency, not
+// by the FP64 pipe, and their sweeps ran slower with the branch-free split (y/z
+// at 128^3 Lax-Friedrichs + MDCD: 76 us, 85 with it; WENO5: 2.1 -> 1.1 ms at 256^3).
+template <int FVS, int RC, int N1, int N2, int N3>
+__device__ __forceinline__ void split_fp64(const DevParams& P, double y2g, const double* raw,
+                                           double Fp[5], double Fm[5]) {
+    if constexpr (RC == RC_WENO5 || RC == RC_MDCD_HYBRID)
+        split_exact<FVS, N1, N2, N3>(P, y2g, raw, Fp, Fm);
+    else
+        split_ieee<FVS, N1, N2, N3>(P.gamma, P.sw_eps, raw, Fp, Fm);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,21 +513,10 @@ __device__ __forceinline__ void eigen_LR(double gamma, const double* ua, double 
 // reversal that reconstruct_select applies for the minus flux (:24-31).
 // ---------------------------------------------------------------------------
 
-// a / b for a divisor b known in advance, with y = RN(1/b) precomputed (an IEEE
-// division): Markstein's theorem (P. Markstein, IBM J. Res. Dev. 34(1), 1990)
-// -- if y is 1/b correctly rounded and q is within one ulp of a/b, then
-// r = a - b q is a double (one exact FMA) and RN(q + r y) = RN(a/b). Here
-// q = RN(a y) is within one ulp, so the result equals the IEEE quotient a / b
-// bit for bit (finite a/b in the normal range), in three operations.
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-    const double q = a * y;
-    const double r = fma(-b, q, a);
-    return fma(r, y, q);
-}
-
-// weno5_reconstruction (reconstruction.cpp:93-124): WENO5-JS, eps 1e-6, p = 2.
+// weno5_reconstruction (reconstruction.cpp:93-124): WENO5-JS, eps 1e-6, p = 2,
+// with the compiler's IEEE divisions: the fallback of the double form below.
 template <class R>
-__device__ __forceinline__ R weno5(R f0, R f1, R f2, R f3, R f4) {
+__device__ __forceinline__ R weno5_ieee(R f0, R f1, R f2, R f3, R f4) {
     const R eps = R(1e-6);
     R beta0 = R(13.0 / 12.0) * (f0 - R(2) * f1 + f2) * (f0 - R(2) * f1 + f2)
             + R(0.25) * (f0 - R(4) * f1 + R(3) * f2) * (f0 - R(4) * f1 + R(3) * f2);
@@ -374,6 +536,42 @@ __device__ __forceinline__ R weno5(R f0, R f1, R f2, R f3, R f4) {
     R p0 = div_rcp(R(2) * f0 - R(7) * f1 + R(11) * f2, six, rcp6);
     R p1 = div_rcp(-f1 + R(5) * f2 + R(2) * f3, six, rcp6);
     R p2 = div_rcp(R(2) * f2 + R(5) * f3 - f4, six, rcp6);
+    return w0 * p0 + w1 * p1 + w2 * p2;
+}
+
+// FP64 form of weno5: the values of weno5_ieee<double> without a branch, so
+// that the ten reconstructions of a face interleave in one scheduling region
+// (the compiler's double division ends the region with its slow path). Two
+// rewrites, both keeping every rounding:
+//   * quotients by div_rcp on a reciprocal from rcp_cubic: one reciprocal and
+//     three operations each for the alpha_k, one shared reciprocal for the
+//     three weights;
+//   * an FMA wherever one factor is a power of two (the product is exact, so
+//     the FMA rounds what the separate operations round once).
+// A reciprocal whose argument overflowed gives NaN where the IEEE quotient is
+// 0: callers test the face for non-finite values and recompute it with
+// weno5_ieee (see recon_face).
+__device__ __forceinline__ double weno5(double f0, double f1, double f2, double f3, double f4) {
+    const double eps = 1e-6;
+    const double m3 = 3.0 * f2;
+    const double t0 = fma(-2.0, f1, f0) + f2, s0 = fma(-4.0, f1, f0) + m3;
+    const double t1 = fma(-2.0, f2, f1) + f3, s1 = f1 - f3;
+    const double t2 = fma(-2.0, f3, f2) + f4, s2 = fma(-4.0, f3, m3) + f4;
+    const double c = 13.0 / 12.0;
+    const double z0 = eps + fma(0.25, s0 * s0, c * t0 * t0);
+    const double z1 = eps + fma(0.25, s1 * s1, c * t1 * t1);
+    const double z2 = eps + fma(0.25, s2 * s2, c * t2 * t2);
+    const double y0 = z0 * z0, y1 = z1 * z1, y2 = z2 * z2;
+    const double a0 = div_rcp(0.1, y0, rcp_cubic(y0));
+    const double a1 = div_rcp(0.6, y1, rcp_cubic(y1));
+    const double a2 = div_rcp(0.3, y2, rcp_cubic(y2));
+    const double as = a0 + a1 + a2;
+    const double ys = rcp_cubic(as);
+    const double w0 = div_rcp(a0, as, ys), w1 = div_rcp(a1, as, ys), w2 = div_rcp(a2, as, ys);
+    const double rcp6 = 1.0 / 6.0;
+    const double p0 = div_rcp(fma(2.0, f0, -(7.0 * f1)) + 11.0 * f2, 6.0, rcp6);
+    const double p1 = div_rcp(fma(2.0, f3, 5.0 * f2 - f1), 6.0, rcp6);
+    const double p2 = div_rcp(fma(2.0, f2, 5.0 * f3) - f4, 6.0, rcp6);
     return w0 * p0 + w1 * p1 + w2 * p2;
 }
 
@@ -520,6 +718,15 @@ __device__ __forceinline__ R mdcd_hybrid(const R* s, const R* lin6, R disp, R di
     return (aa0 * q0 + aa1 * q1 + aa2 * q2 + aa3 * q3) / (aa0 + aa1 + aa2 + aa3);
 }
 
+// Whether any of a face's five values is infinite or NaN (integer tests: the
+// FP64 pipe is what bounds the callers).
+__device__ __forceinline__ bool any_nonfinite(const double* a) {
+    int m = 0;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) m = max(m, __double2hiint(a[q]) & 0x7fffffff);
+    return m >= 0x7ff00000;
+}
+
 // One reconstruction of a window s[0..S-1] (already oriented).
 template <class R, int RC>
 __device__ __forceinline__ R reconstruct(const R* s, const R* lin, R disp, R diss) {
@@ -535,6 +742,44 @@ __device__ __forceinline__ R reconstruct(const R* s, const R* lin, R disp, R dis
     } else {
         return lin[0] * s[0] + lin[1] * s[1] + lin[2] * s[2] + lin[3] * s[3] + lin[4] * s[4] +
                lin[5] * s[5] + lin[6] * s[6] + lin[7] * s[7];
+    }
+}
+
+// The face values of the five components from their windows: P(m, q) / M(m, q)
+// return component q at window position m of F+ / of F- (reversed already, as
+// reconstruct_select does for flag < 0). FP64 WENO5: the branch-free form, and
+// once more by weno5_ieee when a value comes out infinite or NaN, so that
+// overflowing windows give what the IEEE divisions give (a window that holds
+// an infinity is NaN either way). DYN: P and M take a loop variable there (a
+// window in shared memory; one in registers needs q at compile time).
+template <class R, int RC, bool DYN, class GP, class GM>
+__device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R diss, R face[5]) {
+    constexpr int S = Stencil<RC>::S;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        R a[S], b[S];
+#pragma unroll
+        for (int m = 0; m < S; ++m) {
+            a[m] = P(m, q);
+            b[m] = M(m, q);
+        }
+        const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
+        const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
+        face[q] = plus_face + minus_face;
+    }
+    if constexpr (sizeof(R) == 8 && RC == RC_WENO5) {
+        if (any_nonfinite(face)) {
+#pragma unroll(DYN ? 1 : 5)
+            for (int q = 0; q < 5; ++q) {
+                const R f = weno5_ieee<R>(P(0, q), P(1, q), P(2, q), P(3, q), P(4, q)) +
+                            weno5_ieee<R>(M(0, q), M(1, q), M(2, q), M(3, q), M(4, q));
+                if (q == 0) face[0] = f;
+                else if (q == 1) face[1] = f;
+                else if (q == 2) face[2] = f;
+                else if (q == 3) face[3] = f;
+                else face[4] = f;
+            }
+        }
     }
 }
 

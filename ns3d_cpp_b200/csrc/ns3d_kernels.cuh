@@ -94,6 +94,11 @@ __device__ __forceinline__ void char_face(double gamma, const double* wl, const 
         const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
         const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
         wc[q] = plus_face + minus_face;
+        if constexpr (sizeof(R) == 8 && RC == RC_WENO5) {  // as in recon_face
+            if ((__double2hiint(wc[q]) & 0x7ff00000) == 0x7ff00000)
+                wc[q] = weno5_ieee<R>(a[0], a[1], a[2], a[3], a[4]) +
+                        weno5_ieee<R>(b[0], b[1], b[2], b[3], b[4]);
+        }
     }
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
@@ -235,7 +240,6 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
     if (c0 >= len) return;
     const int c1 = min(c0 + seg, len);
 
-    const R gamma = R(P.gamma), eps = R(P.sw_eps);
     R lin[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) lin[m] = R(P.lin[m]);
@@ -255,6 +259,8 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
+    const double y2g = 1.0 / (2.0 * P.gamma);
+    (void)y2g;
     // Loads of one cell's primitives are issued a step before the cell is
     // split (`load_raw` into registers), so their latency hides behind the
     // reconstruction of the current face instead of stalling the march.
@@ -268,15 +274,7 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
     };
     auto split_raw = [&](const double* raw, R* Fp, R* Fm, bool set_ref) {
         if constexpr (!kDeviation) {
-            R rr = R(raw[0]);
-            const R u = R(raw[1]), v = R(raw[2]), w = R(raw[3]), p = R(raw[4]);
-            if (rr <= R(0)) rr = R(1e-12);
-            R E, c;
-            p2c_Ec(rr, u, v, w, p, gamma, E, c);
-            if constexpr (FVS == FV_SW)
-                split_sw<R, DIR == 0, DIR == 1, DIR == 2>(rr, u, v, w, E, p, c, gamma, eps, Fp, Fm);
-            else
-                split_lf<R, DIR == 0, DIR == 1, DIR == 2>(rr, u, v, w, E, p, c, Fp, Fm);
+            split_fp64<FVS, RC, DIR == 0, DIR == 1, DIR == 2>(P, y2g, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, DIR == 0, DIR == 1, DIR == 2>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
@@ -294,8 +292,6 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
             }
         }
     };
-    (void)gamma;
-    (void)eps;
     // CHR: the face's two cells are reloaded (L1/L2 hits); rho as stored.
     auto char_face_at = [&](int f, R* face) {
         double wl[5], wr[5];
@@ -338,18 +334,9 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
             weno5_face_x2([&](int m, int q) { return fp[m][q]; },
                           [&](int m, int q) { return fm[S - 1 - m][q]; }, face);
         } else {
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                R a[S], b[S];
-#pragma unroll
-                for (int m = 0; m < S; ++m) {
-                    a[m] = fp[m][q];
-                    b[m] = fm[S - 1 - m][q];  // reconstruct_select reverses for flag < 0
-                }
-                const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
-                const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
-                face[q] = plus_face + minus_face;
-            }
+            // reconstruct_select reverses for flag < 0
+            recon_face<R, RC, false>([&](int m, int q) { return fp[m][q]; },
+                                     [&](int m, int q) { return fm[S - 1 - m][q]; }, lin, disp, diss, face);
         }
         if (t > 0) {
 #pragma unroll
@@ -583,18 +570,17 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
     const long long n = P.n;
     const long long base = row * nx;
     const int nch = nx >> 5;
-    const R gamma = R(P.gamma), eps = R(P.sw_eps);
     R lin[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) lin[m] = R(P.lin[m]);
     const R disp = R(P.mdcd_disp), diss = R(P.mdcd_diss);
     const R inv_h = R(P.inv_dx);
-    (void)gamma;
-    (void)eps;
 
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
+    const double y2g = 1.0 / (2.0 * P.gamma);
+    (void)y2g;
     auto load_raw = [&](int chunk, double* raw) {
         const long long id = base + (chunk << 5) + lane;
         raw[0] = W.rho[id];
@@ -605,13 +591,7 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
     };
     auto split_raw = [&](const double* raw, R* Fp, R* Fm) {
         if constexpr (!kDeviation) {
-            R rr = R(raw[0]);
-            const R u = R(raw[1]), v = R(raw[2]), w = R(raw[3]), p = R(raw[4]);
-            if (rr <= R(0)) rr = R(1e-12);
-            R E, c;
-            p2c_Ec(rr, u, v, w, p, gamma, E, c);
-            if constexpr (FVS == FV_SW) split_sw<R, 1, 0, 0>(rr, u, v, w, E, p, c, gamma, eps, Fp, Fm);
-            else split_lf<R, 1, 0, 0>(rr, u, v, w, E, p, c, Fp, Fm);
+            split_fp64<FVS, RC, 1, 0, 0>(P, y2g, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, 1, 0, 0>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
@@ -666,18 +646,9 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
             }
         } else {
             // scalar reconstructions: one component of the window at a time
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                R a[S], b[S];
-#pragma unroll
-                for (int m = 0; m < S; ++m) {
-                    a[m] = ring.comp(wq, cell[m], q, false);
-                    b[m] = ring.comp(wq, cell[S - 1 - m], q, true);
-                }
-                const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
-                const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
-                face[q] = plus_face + minus_face;
-            }
+            recon_face<R, RC, true>([&](int m, int q) { return ring.comp(wq, cell[m], q, false); },
+                                    [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); },
+                                          lin, disp, diss, face);
         }
     };
 
@@ -1508,12 +1479,11 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     for (int m = 0; m < 8; ++m) lin[m] = R(P.lin[m]);
     const R disp = R(P.mdcd_disp), diss = R(P.mdcd_diss);
     const R inv_h = R(DIR == 1 ? P.inv_dy : P.inv_dz);
-    const R gamma = R(P.gamma), eps = R(P.sw_eps);
-    (void)gamma;
-    (void)eps;
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
+    const double y2g = 1.0 / (2.0 * P.gamma);
+    (void)y2g;
     auto load_raw = [&](int s, double* raw) {
         const long long id = base + (long long)wrap1(s, len) * stride;
         raw[0] = W.rho[id];
@@ -1526,15 +1496,7 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     // cell's split flux, rounded to float)
     auto split_raw = [&](const double* raw, R* Fp, R* Fm, bool set_ref) {
         if constexpr (!kDeviation) {
-            R rr = R(raw[0]);
-            const R u = R(raw[1]), v = R(raw[2]), w = R(raw[3]), p = R(raw[4]);
-            if (rr <= R(0)) rr = R(1e-12);
-            R E, c;
-            p2c_Ec(rr, u, v, w, p, gamma, E, c);
-            if constexpr (FVS == FV_SW)
-                split_sw<R, 0, DIR == 1, DIR == 2>(rr, u, v, w, E, p, c, gamma, eps, Fp, Fm);
-            else
-                split_lf<R, 0, DIR == 1, DIR == 2>(rr, u, v, w, E, p, c, Fp, Fm);
+            split_fp64<FVS, RC, 0, DIR == 1, DIR == 2>(P, y2g, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, 0, DIR == 1, DIR == 2>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
@@ -1597,18 +1559,9 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
                 int sl[S];
 #pragma unroll
                 for (int m = 0; m < S; ++m) sl[m] = ph + m < S ? ph + m : ph + m - S;
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    R a[S], b[S];
-#pragma unroll
-                    for (int m = 0; m < S; ++m) {
-                        a[m] = ring.comp(sl[m], tid, q, false);
-                        b[m] = ring.comp(sl[S - 1 - m], tid, q, true);
-                    }
-                    const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
-                    const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
-                    face[q] = plus_face + minus_face;
-                }
+                recon_face<R, RC, true>([&](int m, int q) { return ring.comp(sl[m], tid, q, false); },
+                                        [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); },
+                                              lin, disp, diss, face);
             }
             if (t > 0) {
                 R tz[5];
