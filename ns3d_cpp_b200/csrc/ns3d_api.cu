@@ -768,6 +768,7 @@ ns3d_status build_launch_cfg(const ns3d_params* p, LaunchCfg* L, std::string* ms
     linear_coefficients(q, P.lin);
     P.mdcd_disp = q.mdcd_disp; P.mdcd_diss = q.mdcd_diss;
     P.vis_order = q.vis_scheme == NS3D_VIS_C4TH ? 4 : (q.vis_scheme == NS3D_VIS_C6TH ? 6 : 8);
+    derive_quotients(P);
     L->fvs = q.fvs_type == NS3D_FVS_STEGER_WARMING ? FV_SW : FV_LF;
     L->rc = recon_kind(q.recon);
     L->chr = q.char_recon ? 1 : 0;
@@ -816,6 +817,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     linear_coefficients(q, P.lin);
     P.mdcd_disp = q.mdcd_disp; P.mdcd_diss = q.mdcd_diss;
     P.vis_order = q.vis_scheme == NS3D_VIS_C4TH ? 4 : (q.vis_scheme == NS3D_VIS_C6TH ? 6 : 8);
+    derive_quotients(P);
     ctx->L.fvs = q.fvs_type == NS3D_FVS_STEGER_WARMING ? FV_SW : FV_LF;
     ctx->L.rc = recon_kind(q.recon);
     ctx->L.chr = q.char_recon ? 1 : 0;

@@ -38,7 +38,23 @@ struct DevParams {
     double lin[8];   // linear reconstruction coefficients (LIN6 / LIN8)
     double mdcd_disp, mdcd_diss;
     int vis_order;   // 4, 6, 8
+    // divisors of the central derivatives (12 h, 60 h or h) along x, y, z, and
+    // the reciprocals RN(1/b) of these, of the heat flux's Pr and of the
+    // split's 2 gamma (see quot_rcp)
+    double dd[3], rdd[3], rPr, r2g;
 };
+
+// The derived constants above, from the fields before them.
+inline void derive_quotients(DevParams& P) {
+    const double c = P.vis_order == 4 ? 12.0 : (P.vis_order == 6 ? 60.0 : 1.0);
+    const double h[3] = {P.dx, P.dy, P.dz};
+    for (int d = 0; d < 3; ++d) {
+        P.dd[d] = c * h[d];
+        P.rdd[d] = 1.0 / P.dd[d];
+    }
+    P.rPr = 1.0 / P.Pr;
+    P.r2g = 1.0 / (2.0 * P.gamma);
+}
 
 // ---------------------------------------------------------------------------
 // IEEE quotients and square roots without a branch
@@ -96,6 +112,27 @@ __device__ __forceinline__ bool mid_range(double x) {
 __device__ __forceinline__ bool finite_hi(double x) {
     return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
+// a / b: div_rcp where its range allows (b mid-range, quotient finite), else
+// the compiler's division out of line.
+static __device__ __noinline__ double div_cold(double a, double b) { return a / b; }
+__device__ __forceinline__ double quot_mid(double a, double b) {
+    const double q = div_rcp(a, b, rcp_cubic(b));
+    return mid_range(b) && finite_hi(q) ? q : div_cold(a, b);
+}
+static __device__ __noinline__ double sqrt_cold(double b) { return sqrt(b); }
+__device__ __forceinline__ double sqrt_mid(double b) {
+    const double s = sqrt_cubic(b);
+    return mid_range(b) ? s : sqrt_cold(b);
+}
+
+// a / b for a constant b > 0 with y = RN(1/b): div_rcp, keeping the infinities
+// and NaN of the IEEE quotient (its residual would turn them into NaN).
+__device__ __forceinline__ double quot_rcp(double a, double b, double y) {
+    const double q = a * y;
+    const double r = fma(fma(-b, q, a), y, q);
+    return finite_hi(q) ? r : q;
+}
+
 // ---------------------------------------------------------------------------
 // Thermodynamics (field_structures.h:94-105, 405-451)
 // ---------------------------------------------------------------------------
@@ -125,6 +162,24 @@ __device__ __forceinline__ double pow_1p5(double T) {
 template <class R>
 __device__ __forceinline__ R get_mu(R T, R mu_ref, R S) {
     return mu_ref * pow_1p5(T) * (R(1.0) + S) / (T + S);
+}
+static __device__ __noinline__ double get_mu_cold(double T, double mu_ref, double S) {
+    return get_mu<double>(T, mu_ref, S);
+}
+
+// get_mu<double>'s value with its square root and quotient branch-free;
+// temperatures outside the mid range (zero, negative and NaN among them) take
+// get_mu itself.
+__device__ __forceinline__ double get_mu_exact(double T, double mu_ref, double S) {
+    const double s = sqrt_cubic(T);
+    const double r = fma(-s, s, T);
+    const double p = T * s;
+    const double e = fma(T, s, -p);
+    const double p15 = p + (e + 0.5 * (r * s));
+    const double TS = T + S;
+    const double q = div_rcp(mu_ref * p15 * (1.0 + S), TS, rcp_cubic(TS));
+    if (mid_range(T) && mid_range(TS) && finite_hi(q)) return q;
+    return get_mu_cold(T, mu_ref, S);
 }
 
 // FP32-stencil form: T^1.5 as T sqrt(T) (the difference from pow is far below
@@ -238,9 +293,9 @@ __device__ __noinline__ void split_ieee_cold(double gamma, double eps, const dou
 // constant's), the products with the zero components of the normal left out
 // (they add a zero) and 0.5 (l +- |l|) as the selection it is. States outside
 // the ranges those need take split_ieee: density, pressure or sound speed extreme or not
-// a number, energy not finite. y2g = RN(1 / (2 gamma)).
+// a number, energy not finite.
 template <int FVS, int N1, int N2, int N3>
-__device__ __forceinline__ void split_exact(const DevParams& P, double y2g, const double* raw,
+__device__ __forceinline__ void split_exact(const DevParams& P, const double* raw,
                                             double Fp[5], double Fm[5]) {
     static_assert(N1 + N2 + N3 == 1, "axis-aligned face normal");
     const double gamma = P.gamma, eps = P.sw_eps;
@@ -274,7 +329,7 @@ __device__ __forceinline__ void split_exact(const DevParams& P, double y2g, cons
         }
         const double S1p = l1p + l3p, S1m = l1m + l3m, S2p = l3p - l1p, S2m = l3m - l1m;
         const double H = div_rcp(E + p, rho, yr);
-        const double ga1 = div_rcp(rho, 2.0 * gamma, y2g), ga2 = 2.0 * (gamma - 1.0);
+        const double ga1 = div_rcp(rho, 2.0 * gamma, P.r2g), ga2 = 2.0 * (gamma - 1.0);
         const double gp = ga2 * l2p, gm = ga2 * l2m;
         const double cp = S2p * c, cm = S2m * c;
         const double vel[3] = {u, v, w};
@@ -320,10 +375,10 @@ __device__ __forceinline__ void split_exact(const DevParams& P, double y2g, cons
 // by the FP64 pipe, and their sweeps ran slower with the branch-free split (y/z
 // at 128^3 Lax-Friedrichs + MDCD: 76 us, 85 with it; WENO5: 2.1 -> 1.1 ms at 256^3).
 template <int FVS, int RC, int N1, int N2, int N3>
-__device__ __forceinline__ void split_fp64(const DevParams& P, double y2g, const double* raw,
-                                           double Fp[5], double Fm[5]) {
+__device__ __forceinline__ void split_fp64(const DevParams& P, const double* raw, double Fp[5],
+                                           double Fm[5]) {
     if constexpr (RC == RC_WENO5 || RC == RC_MDCD_HYBRID)
-        split_exact<FVS, N1, N2, N3>(P, y2g, raw, Fp, Fm);
+        split_exact<FVS, N1, N2, N3>(P, raw, Fp, Fm);
     else
         split_ieee<FVS, N1, N2, N3>(P.gamma, P.sw_eps, raw, Fp, Fm);
 }
@@ -798,6 +853,28 @@ __device__ __forceinline__ R dcentral(F f, R h) {
         const R c1 = R(0.8), c2 = R(-0.2), c3 = R(0.0380952380952381), c4 = R(-0.00357142857142857);
         return (c1 * (f(1) - f(-1)) + c2 * (f(2) - f(-2)) + c3 * (f(3) - f(-3)) +
                 c4 * (f(4) - f(-4))) / h;
+    }
+}
+
+// The same derivative along x, y or z (dir 0, 1, 2; spacing h) of a box: the FP64 form's
+// division by the constant divisor as quot_rcp (the IEEE quotient; twelve per
+// cell in the viscous flux and twelve in its divergence).
+template <class R, int ORD, class F>
+__device__ __forceinline__ R dcentral_dir(const DevParams& P, int dir, F f, R h) {
+    if constexpr (sizeof(R) == 8) {
+        // dcentral's numerators
+        double x;
+        if constexpr (ORD == 4) {
+            x = fma(-8.0, f(-1), fma(8.0, f(1), -f(2))) + f(-2);  // 8 f is exact
+        } else if constexpr (ORD == 6) {
+            x = f(3) - 9.0 * f(2) + 45.0 * f(1) - 45.0 * f(-1) + 9.0 * f(-2) - f(-3);
+        } else {
+            const double c1 = 0.8, c2 = -0.2, c3 = 0.0380952380952381, c4 = -0.00357142857142857;
+            x = c1 * (f(1) - f(-1)) + c2 * (f(2) - f(-2)) + c3 * (f(3) - f(-3)) + c4 * (f(4) - f(-4));
+        }
+        return quot_rcp(x, P.dd[dir], P.rdd[dir]);
+    } else {
+        return dcentral<R, ORD>(f, h);
     }
 }
 

@@ -259,8 +259,6 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
-    const double y2g = 1.0 / (2.0 * P.gamma);
-    (void)y2g;
     // Loads of one cell's primitives are issued a step before the cell is
     // split (`load_raw` into registers), so their latency hides behind the
     // reconstruction of the current face instead of stalling the march.
@@ -274,7 +272,7 @@ k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __r
     };
     auto split_raw = [&](const double* raw, R* Fp, R* Fm, bool set_ref) {
         if constexpr (!kDeviation) {
-            split_fp64<FVS, RC, DIR == 0, DIR == 1, DIR == 2>(P, y2g, raw, Fp, Fm);
+            split_fp64<FVS, RC, DIR == 0, DIR == 1, DIR == 2>(P, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, DIR == 0, DIR == 1, DIR == 2>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
@@ -579,8 +577,6 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
-    const double y2g = 1.0 / (2.0 * P.gamma);
-    (void)y2g;
     auto load_raw = [&](int chunk, double* raw) {
         const long long id = base + (chunk << 5) + lane;
         raw[0] = W.rho[id];
@@ -591,7 +587,7 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
     };
     auto split_raw = [&](const double* raw, R* Fp, R* Fm) {
         if constexpr (!kDeviation) {
-            split_fp64<FVS, RC, 1, 0, 0>(P, y2g, raw, Fp, Fm);
+            split_fp64<FVS, RC, 1, 0, 0>(P, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, 1, 0, 0>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
@@ -747,6 +743,19 @@ __device__ __forceinline__ void store_fv(R* fv, long long n, long long id, R txx
     }
 }
 
+// get_mu of the form (FP64: get_mu_exact, the same value branch-free) and the
+// heat flux's mu Cp / Pr.
+template <class R>
+__device__ __forceinline__ R mu_of(R T, R mu_ref, R S) {
+    if constexpr (sizeof(R) == 8) return get_mu_exact(T, mu_ref, S);
+    else return get_mu<R>(T, mu_ref, S);
+}
+template <class R>
+__device__ __forceinline__ R heat_coef(const DevParams& P, R mu, R Cp, R Pr) {
+    if constexpr (sizeof(R) == 8) return quot_rcp(mu * Cp, Pr, P.rPr);
+    else return mu * Cp / Pr;
+}
+
 // ---------------------------------------------------------------------------
 // Viscous flux (compute_gradients ViscousFlux.cpp:240-279 +
 // compute_viscous_flux :282-339). Output fv (type R) in the layout of store_fv:
@@ -782,21 +791,22 @@ k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict
         return [=](int o) { return R(a[id + (long long)(wrap1(k + o, nz) - k) * sxy] - c0); };
     };
     const R dx = R(P.dx), dy = R(P.dy), dz = R(P.dz);
-    const R du_dx = dcentral<R, ORD>(gx(W.u), dx);
-    const R du_dy = dcentral<R, ORD>(gy(W.u), dy);
-    const R du_dz = dcentral<R, ORD>(gz(W.u), dz);
-    const R dv_dx = dcentral<R, ORD>(gx(W.v), dx);
-    const R dv_dy = dcentral<R, ORD>(gy(W.v), dy);
-    const R dv_dz = dcentral<R, ORD>(gz(W.v), dz);
-    const R dw_dx = dcentral<R, ORD>(gx(W.w), dx);
-    const R dw_dy = dcentral<R, ORD>(gy(W.w), dy);
-    const R dw_dz = dcentral<R, ORD>(gz(W.w), dz);
-    const R dT_dx = dcentral<R, ORD>(gx(W.T), dx);
-    const R dT_dy = dcentral<R, ORD>(gy(W.T), dy);
-    const R dT_dz = dcentral<R, ORD>(gz(W.T), dz);
+    const R du_dx = dcentral_dir<R, ORD>(P, 0, gx(W.u), dx);
+    const R du_dy = dcentral_dir<R, ORD>(P, 1, gy(W.u), dy);
+    const R du_dz = dcentral_dir<R, ORD>(P, 2, gz(W.u), dz);
+    const R dv_dx = dcentral_dir<R, ORD>(P, 0, gx(W.v), dx);
+    const R dv_dy = dcentral_dir<R, ORD>(P, 1, gy(W.v), dy);
+    const R dv_dz = dcentral_dir<R, ORD>(P, 2, gz(W.v), dz);
+    const R dw_dx = dcentral_dir<R, ORD>(P, 0, gx(W.w), dx);
+    const R dw_dy = dcentral_dir<R, ORD>(P, 1, gy(W.w), dy);
+    const R dw_dz = dcentral_dir<R, ORD>(P, 2, gz(W.w), dz);
+    const R dT_dx = dcentral_dir<R, ORD>(P, 0, gx(W.T), dx);
+    const R dT_dy = dcentral_dir<R, ORD>(P, 1, gy(W.T), dy);
+    const R dT_dz = dcentral_dir<R, ORD>(P, 2, gz(W.T), dz);
 
-    const R mu = get_mu<R>(R(W.T[id]), R(P.mu), R(P.sutherland_s));
+    const R mu = mu_of<R>(R(W.T[id]), R(P.mu), R(P.sutherland_s));
     const R Cp = R(P.Cp), Pr = R(P.Pr);
+    const R kq = heat_coef<R>(P, mu, Cp, Pr);
     const R divU = du_dx + dv_dy + dw_dz;
     const R tau_xx = R(2.0) * mu * du_dx - R(2.0 / 3.0) * mu * divU;
     const R tau_yy = R(2.0) * mu * dv_dy - R(2.0 / 3.0) * mu * divU;
@@ -804,9 +814,9 @@ k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict
     const R tau_xy = mu * (du_dy + dv_dx);
     const R tau_xz = mu * (du_dz + dw_dx);
     const R tau_yz = mu * (dv_dz + dw_dy);
-    const R qx = mu * Cp / Pr * dT_dx;
-    const R qy = mu * Cp / Pr * dT_dy;
-    const R qz = mu * Cp / Pr * dT_dz;
+    const R qx = kq * dT_dx;
+    const R qy = kq * dT_dy;
+    const R qz = kq * dT_dz;
     const R u = R(W.u[id]), v = R(W.v[id]), w = R(W.w[id]);
     store_fv<R>(fv, n, id, tau_xx, tau_yy, tau_zz, tau_xy, tau_xz, tau_yz,
                 u * tau_xx + v * tau_xy + w * tau_xz + qx, u * tau_xy + v * tau_yy + w * tau_yz + qy,
@@ -885,15 +895,16 @@ k_visc_flux_25d(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __rest
         R g[4][3];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            g[v][0] = dcentral<R, ORD>([&](int o) { return tile[v][cy][cx + o]; }, dx);
-            g[v][1] = dcentral<R, ORD>([&](int o) { return tile[v][cy + o][cx]; }, dy);
-            g[v][2] = dcentral<R, ORD>([&](int o) { return q[v][4 + o]; }, dz);
+            g[v][0] = dcentral_dir<R, ORD>(P, 0, [&](int o) { return tile[v][cy][cx + o]; }, dx);
+            g[v][1] = dcentral_dir<R, ORD>(P, 1, [&](int o) { return tile[v][cy + o][cx]; }, dy);
+            g[v][2] = dcentral_dir<R, ORD>(P, 2, [&](int o) { return q[v][4 + o]; }, dz);
         }
         const R du_dx = g[0][0], du_dy = g[0][1], du_dz = g[0][2];
         const R dv_dx = g[1][0], dv_dy = g[1][1], dv_dz = g[1][2];
         const R dw_dx = g[2][0], dw_dy = g[2][1], dw_dz = g[2][2];
         const R dT_dx = g[3][0], dT_dy = g[3][1], dT_dz = g[3][2];
-        const R mu = get_mu<R>(R(ref[3]) + q[3][4], mu_ref, Ss);
+        const R mu = mu_of<R>(R(ref[3]) + q[3][4], mu_ref, Ss);
+        const R kq = heat_coef<R>(P, mu, Cp, Pr);
         const R divU = du_dx + dv_dy + dw_dz;
         const R tau_xx = R(2.0) * mu * du_dx - R(2.0 / 3.0) * mu * divU;
         const R tau_yy = R(2.0) * mu * dv_dy - R(2.0 / 3.0) * mu * divU;
@@ -901,9 +912,9 @@ k_visc_flux_25d(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __rest
         const R tau_xy = mu * (du_dy + dv_dx);
         const R tau_xz = mu * (du_dz + dw_dx);
         const R tau_yz = mu * (dv_dz + dw_dy);
-        const R qx = mu * Cp / Pr * dT_dx;
-        const R qy = mu * Cp / Pr * dT_dy;
-        const R qz = mu * Cp / Pr * dT_dz;
+        const R qx = kq * dT_dx;
+        const R qy = kq * dT_dy;
+        const R qz = kq * dT_dz;
         const R u = R(ref[0]) + q[0][4], v = R(ref[1]) + q[1][4], w = R(ref[2]) + q[2][4];
         const long long id = plane + col;
         store_fv<R>(fv, n, id, tau_xx, tau_yy, tau_zz, tau_xy, tau_xz, tau_yz,
@@ -1106,17 +1117,18 @@ k_visc_flux_pipe(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __res
         } else {
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-                g[v][0] = dcentral<R, ORD>([&](int o) { return tile[b][v][cy][cx + o]; }, dx);
-                g[v][1] = dcentral<R, ORD>([&](int o) { return tile[b][v][cy + o][cx]; }, dy);
+                g[v][0] = dcentral_dir<R, ORD>(P, 0, [&](int o) { return tile[b][v][cy][cx + o]; }, dx);
+                g[v][1] = dcentral_dir<R, ORD>(P, 1, [&](int o) { return tile[b][v][cy + o][cx]; }, dy);
             }
         }
 #pragma unroll
-        for (int v = 0; v < 4; ++v) g[v][2] = dcentral<R, ORD>([&](int o) { return q[v][4 + o]; }, dz);
+        for (int v = 0; v < 4; ++v) g[v][2] = dcentral_dir<R, ORD>(P, 2, [&](int o) { return q[v][4 + o]; }, dz);
         const R du_dx = g[0][0], du_dy = g[0][1], du_dz = g[0][2];
         const R dv_dx = g[1][0], dv_dy = g[1][1], dv_dz = g[1][2];
         const R dw_dx = g[2][0], dw_dy = g[2][1], dw_dz = g[2][2];
         const R dT_dx = g[3][0], dT_dy = g[3][1], dT_dz = g[3][2];
-        const R mu = get_mu<R>(R(ref[3]) + q[3][4], mu_ref, Ss);
+        const R mu = mu_of<R>(R(ref[3]) + q[3][4], mu_ref, Ss);
+        const R kq = heat_coef<R>(P, mu, Cp, Pr);
         const R divU = du_dx + dv_dy + dw_dz;
         const R tau_xx = R(2.0) * mu * du_dx - R(2.0 / 3.0) * mu * divU;
         const R tau_yy = R(2.0) * mu * dv_dy - R(2.0 / 3.0) * mu * divU;
@@ -1124,9 +1136,9 @@ k_visc_flux_pipe(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __res
         const R tau_xy = mu * (du_dy + dv_dx);
         const R tau_xz = mu * (du_dz + dw_dx);
         const R tau_yz = mu * (dv_dz + dw_dy);
-        const R qx = mu * Cp / Pr * dT_dx;
-        const R qy = mu * Cp / Pr * dT_dy;
-        const R qz = mu * Cp / Pr * dT_dz;
+        const R qx = kq * dT_dx;
+        const R qy = kq * dT_dy;
+        const R qz = kq * dT_dz;
         const R u = R(ref[0]) + q[0][4], v = R(ref[1]) + q[1][4], w = R(ref[2]) + q[2][4];
         const long long id = (long long)k * sxy + col;
         store_fv<R>(fv, n, id, tau_xx, tau_yy, tau_zz, tau_xy, tau_xz, tau_yz,
@@ -1192,9 +1204,9 @@ __device__ __forceinline__ void cell_visc(const DevParams& P, const R* __restric
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             R acc = R(0.0);
-            acc += dcentral<R, ORD>(gx(FX[m]), dx);
-            acc += dcentral<R, ORD>(gy(FY[m]), dy);
-            acc += dcentral<R, ORD>(gz(FZ[m]), dz);
+            acc += dcentral_dir<R, ORD>(P, 0, gx(FX[m]), dx);
+            acc += dcentral_dir<R, ORD>(P, 1, gy(FY[m]), dy);
+            acc += dcentral_dir<R, ORD>(P, 2, gz(FZ[m]), dz);
             r[m + 1] = acc;
         }
     }
@@ -1238,7 +1250,7 @@ __device__ __forceinline__ void prim2cons_cell(const StateView& W, long long id,
     U[2] = rr * v;
     U[3] = rr * w;
     const double kinetic = 0.5 * (u * u + v * v + w * w);
-    const double e_internal = p / ((gamma - 1.0) * rr);
+    const double e_internal = quot_mid(p, (gamma - 1.0) * rr);
     U[4] = rr * (e_internal + kinetic);
 }
 
@@ -1246,10 +1258,10 @@ __device__ __forceinline__ void prim2cons_cell(const StateView& W, long long id,
 // semantics (a NaN candidate never replaces the running minimum).
 __device__ __forceinline__ double cfl_candidate(const DevParams& P, double rho, double u,
                                                 double v, double w, double p) {
-    const double a = sqrt(P.gamma * p / (rho < 1e-14 ? 1e-14 : rho));
-    const double dt_x = P.dx / (fabs(u) + a);
-    const double dt_y = P.dy / (fabs(v) + a);
-    const double dt_z = P.dz / (fabs(w) + a);
+    const double a = sqrt_mid(quot_mid(P.gamma * p, rho < 1e-14 ? 1e-14 : rho));
+    const double dt_x = quot_mid(P.dx, fabs(u) + a);
+    const double dt_y = quot_mid(P.dy, fabs(v) + a);
+    const double dt_z = quot_mid(P.dz, fabs(w) + a);
     double m = (dt_z < dt_y) ? dt_z : dt_y;
     m = (m < dt_x) ? m : dt_x;
     return m;
@@ -1344,13 +1356,22 @@ __device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& 
         p = (gamma - 1.0) * (U[4] - rr * (0.5 * (u * u + v * v + w * w)));
         T = p * ir * (1.0 / P.Rgas);
     } else {
-        u = U[1] / rr;
-        v = U[2] / rr;
-        w = U[3] / rr;
+        // U / rr by one reciprocal (the IEEE quotients, see div_rcp)
+        const double yr = rcp_cubic(rr);
+        u = div_rcp(U[1], rr, yr);
+        v = div_rcp(U[2], rr, yr);
+        w = div_rcp(U[3], rr, yr);
+        double e = div_rcp(U[4], rr, yr);
+        if (!mid_range(rr) || !finite_hi(u) || !finite_hi(v) || !finite_hi(w) || !finite_hi(e)) {
+            u = div_cold(U[1], rr);
+            v = div_cold(U[2], rr);
+            w = div_cold(U[3], rr);
+            e = div_cold(U[4], rr);
+        }
         const double kinetic = 0.5 * (u * u + v * v + w * w);
-        const double e_internal = U[4] / rr - kinetic;
+        const double e_internal = e - kinetic;
         p = (gamma - 1.0) * rr * e_internal;
-        T = p / (rr * P.Rgas);  // primitiveToConserved's T
+        T = quot_mid(p, rr * P.Rgas);  // primitiveToConserved's T
     }
     Wn.rho[id] = rr;
     Wn.u[id] = u;
@@ -1482,8 +1503,6 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     double refp[5], refm[5];
     const double inv_gm1 = kDeviation ? 1.0 / (P.gamma - 1.0) : 0.0;
     const double inv_2g = kDeviation ? 1.0 / (2.0 * P.gamma) : 0.0;
-    const double y2g = 1.0 / (2.0 * P.gamma);
-    (void)y2g;
     auto load_raw = [&](int s, double* raw) {
         const long long id = base + (long long)wrap1(s, len) * stride;
         raw[0] = W.rho[id];
@@ -1496,7 +1515,7 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     // cell's split flux, rounded to float)
     auto split_raw = [&](const double* raw, R* Fp, R* Fm, bool set_ref) {
         if constexpr (!kDeviation) {
-            split_fp64<FVS, RC, 0, DIR == 1, DIR == 2>(P, y2g, raw, Fp, Fm);
+            split_fp64<FVS, RC, 0, DIR == 1, DIR == 2>(P, raw, Fp, Fm);
         } else {
             double Fpd[5], Fmd[5];
             split_fast<FVS, 0, DIR == 1, DIR == 2>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
