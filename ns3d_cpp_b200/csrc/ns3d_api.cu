@@ -28,13 +28,13 @@ namespace ns3d {
 extern template cudaError_t launch_sweep<double>(const LaunchCfg&, int, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<double>(const LaunchCfg&, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_update<double>(const LaunchCfg&, int, StateView, StateView,
-                                                  const double*, const double*, StateOut, Ctrl*);
-extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*);
+                                                  const double*, const double*, StateOut, Ctrl*, bool);
+extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*, bool);
 extern template cudaError_t launch_sweep<float>(const LaunchCfg&, int, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<float>(const LaunchCfg&, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_update<float>(const LaunchCfg&, int, StateView, StateView,
-                                                 const float*, const float*, StateOut, Ctrl*);
-extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*);
+                                                 const float*, const float*, StateOut, Ctrl*, bool);
+extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*, bool);
 extern template cudaError_t launch_sweep_z_update<double>(const LaunchCfg&, int, StateView, StateView,
                                                           const double*, const double*, StateOut, Ctrl*);
 extern template cudaError_t launch_sweep_z_update<float>(const LaunchCfg&, int, StateView, StateView,
@@ -58,6 +58,8 @@ struct ns3d_ctx {
     // the z sweep fused with the stage update (NS3D_FUSE=1) or the two kernels
     // (NS3D_FUSE=0); the same bits either way
     bool fuse = false;
+    // FP64 small box: k_flux_small, T_acc as three separate terms (15 n values)
+    bool t3 = false;
     long long n = 0;
     double* wmem = nullptr;      // 3 state buffers x 6 arrays x n
     double* slot[3] = {nullptr, nullptr, nullptr};  // state buffer b: 6 arrays of n from slot[b]
@@ -71,7 +73,7 @@ struct ns3d_ctx {
     const double* pre_h[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool prefetched = false;
     int cur = 0, rec = 0;        // current state buffer, recorded (U0) buffer
-    void* tacc = nullptr;        // 5 n (R)
+    void* tacc = nullptr;        // 5 n (R); 15 n with t3
     void* fv = nullptr;          // viscous fluxes: 9 n doubles (FP64) or 3 n float4 (FP32)
     size_t rsize = 8;            // sizeof(R)
     Ctrl* ctrl = nullptr;
@@ -535,6 +537,12 @@ ns3d_status read_ctrl(ns3d_ctx* ctx) {
 template <class R>
 ns3d_status rhs_parts_t(ns3d_ctx* ctx, StateView W, const Ctrl* ctrl, int dirs = 3) {
     R* tacc = (R*)ctx->tacc;
+    if constexpr (sizeof(R) == 8) {
+        if (ctx->t3) {
+            NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1, launch_flux_small(ctx->L, W, tacc, (R*)ctx->fv, ctrl));
+            return NS3D_OK;
+        }
+    }
     if (ctx->overlap) {
         // the viscous flux (state -> fv) beside the sweeps (state -> T_acc):
         // fork after the work already queued, join before the update
@@ -576,7 +584,7 @@ ns3d_status stage_t(ns3d_ctx* ctx, int stage, StateView Wc, StateView W0, StateO
         ns3d_status s = rhs_parts_t<R>(ctx, Wc, ctx->ctrl);
         if (s != NS3D_OK) return s;
         NS3D_LAUNCH(NS3D_KERNEL_UPDATE, 1,
-                    launch_update<R>(ctx->L, stage, Wc, W0, tacc, fv, Wn, ctx->ctrl));
+                    launch_update<R>(ctx->L, stage, Wc, W0, tacc, fv, Wn, ctx->ctrl, ctx->t3));
         return NS3D_OK;
     }
     ns3d_status s = rhs_parts_t<R>(ctx, Wc, ctx->ctrl, 2);
@@ -739,6 +747,11 @@ void default_tiling(LaunchCfg& L) {
     L.zb = 0;
     L.tiled = 3;  // 2.5-D viscous flux, pipelined plane loads (k_visc_flux_pipe)
     L.pipe = 3;   // FP32 sweeps with the software-pipelined split (k_sweep_x_pipe, k_sweep_pipe)
+    // an override of the marching kernels' shapes selects those kernels
+    L.small = 300000;
+    for (const char* v : {"NS3D_TILE_ZB", "NS3D_TILED", "NS3D_SEG"})
+        if (std::getenv(v)) L.small = 0;
+    if (const char* e = std::getenv("NS3D_SMALL")) L.small = std::atoll(e);
     if (const char* e = std::getenv("NS3D_PIPE")) L.pipe = std::atoi(e);
     if (const char* e = std::getenv("NS3D_TILE_ZB")) L.zb = std::atoi(e);
     if (const char* e = std::getenv("NS3D_TILED")) L.tiled = std::atoi(e);
@@ -843,8 +856,9 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
          cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess))
         return bail(NS3D_ERR_CUDA, "second stream for the overlapped viscous flux");
     const size_t n = (size_t)ctx->n;
+    ctx->t3 = ctx->rsize == sizeof(double) && !ctx->fuse && !ctx->overlap && small_box(ctx->L);
     if (cudaMalloc(&ctx->wmem, sizeof(double) * 18 * n) != cudaSuccess ||
-        cudaMalloc(&ctx->tacc, ctx->rsize * 5 * n) != cudaSuccess ||
+        cudaMalloc(&ctx->tacc, ctx->rsize * (ctx->t3 ? 15 : 5) * n) != cudaSuccess ||
         cudaMalloc(&ctx->fv, ctx->rsize * (ctx->rsize == 4 ? fv_values_per_cell<float>() : fv_values_per_cell<double>()) * n) != cudaSuccess ||
         cudaMalloc(&ctx->ctrl, sizeof(Ctrl)) != cudaSuccess) {
         cudaGetLastError();
@@ -908,7 +922,7 @@ ns3d_status ns3d_get_params(const ns3d_ctx* ctx, ns3d_params* out) {
 ns3d_status ns3d_device_bytes(const ns3d_ctx* ctx, size_t* bytes) {
     if (!ctx || !bytes) return NS3D_ERR_INVALID;
     *bytes = sizeof(double) * (ctx->stage_mem ? 24 : 18) * (size_t)ctx->n +
-             ctx->rsize * 14 * (size_t)ctx->n;
+             ctx->rsize * (ctx->t3 ? 24 : 14) * (size_t)ctx->n;
     for (size_t c : ctx->adj_cap) *bytes += sizeof(double) * c;
     return NS3D_OK;
 }
@@ -1053,10 +1067,10 @@ ns3d_status ns3d_compute_rhs(ns3d_ctx* ctx, double* r0, double* r1, double* r2, 
     double* rhs = warr(ctx, tmpb, 0);
     if (ctx->p.precision == NS3D_PREC_FP64)
         NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    launch_rhs_out<double>(ctx->L, (const double*)ctx->tacc, (const double*)ctx->fv, rhs));
+                    launch_rhs_out<double>(ctx->L, (const double*)ctx->tacc, (const double*)ctx->fv, rhs, ctx->t3));
     else
         NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    launch_rhs_out<float>(ctx->L, (const float*)ctx->tacc, (const float*)ctx->fv, rhs));
+                    launch_rhs_out<float>(ctx->L, (const float*)ctx->tacc, (const float*)ctx->fv, rhs, ctx->t3));
     const double* d[5];
     for (int q = 0; q < 5; ++q) d[q] = rhs + q * ctx->n;
     double* h[5] = {r0, r1, r2, r3, r4};

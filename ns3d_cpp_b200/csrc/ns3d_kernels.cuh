@@ -763,20 +763,17 @@ __device__ __forceinline__ R heat_coef(const DevParams& P, R mu, R Cp, R Pr) {
 // reference's 12 flux arrays map onto these (Fv = {xx, xy, xz, ex},
 // Hv = {xy, yy, yz, ey}, Gv = {xz, yz, zz, ez}); the mass fluxes are zero.
 // ---------------------------------------------------------------------------
+// One cell, neighbours from memory. FP32-stencil form: differentiates
+// deviations from the centre value, formed in double (the central stencils'
+// coefficients sum to zero, so the derivative is unchanged while T ~ 1 +- small
+// keeps its low-order digits).
 template <class R, int ORD>
-__global__ void __launch_bounds__(128)
-k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict__ ctrl) {
-    if (ctrl && ctrl->stop) return;
+__device__ __forceinline__ void visc_cell(const DevParams& P, const StateView& W, R* __restrict__ fv,
+                                          int i, int j, int k) {
     const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
     const long long n = P.n;
     const long long id = ((long long)k * ny + j) * nx + i;
     const long long sxy = (long long)nx * ny;
-    // FP32-stencil form: differentiate deviations from the centre value, formed
-    // in double (the central stencils' coefficients sum to zero, so the
-    // derivative is unchanged while T ~ 1 +- small keeps its low-order digits).
     constexpr bool kDeviation = sizeof(R) < sizeof(double);
     auto gx = [&](const double* a) {
         const double c0 = kDeviation ? a[id] : 0.0;
@@ -821,6 +818,15 @@ k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict
     store_fv<R>(fv, n, id, tau_xx, tau_yy, tau_zz, tau_xy, tau_xz, tau_yz,
                 u * tau_xx + v * tau_xy + w * tau_xz + qx, u * tau_xy + v * tau_yy + w * tau_yz + qy,
                 u * tau_xz + v * tau_yz + w * tau_zz + qz);
+}
+
+template <class R, int ORD>
+__global__ void __launch_bounds__(128)
+k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict__ ctrl) {
+    if (ctrl && ctrl->stop) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.nx) return;
+    visc_cell<R, ORD>(P, W, fv, i, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -1212,20 +1218,29 @@ __device__ __forceinline__ void cell_visc(const DevParams& P, const R* __restric
     }
 }
 
+// T_acc of one cell and component. T3 (FP64 form): from the separate x, y and
+// z terms of k_flux_small (15 blocks of n), added in the marching sweeps' order.
+template <class R, bool T3>
+__device__ __forceinline__ R acc_term(const DevParams& P, const R* __restrict__ tacc, int q, long long id) {
+    static_assert(!T3 || sizeof(R) == 8, "separate terms belong to the FP64 form");
+    const long long n = P.n;
+    if constexpr (T3) return (tacc[q * n + id] + tacc[(5 + q) * n + id]) + tacc[(10 + q) * n + id];
+    else return tacc[q * n + id];
+}
+
 // rhs at one cell: the viscous part followed by the inviscid divergence
 // (range_kutta.cpp:61-97) accumulated in tacc.
-template <class R, int ORD>
+template <class R, int ORD, bool T3>
 __device__ __forceinline__ void cell_rhs(const DevParams& P, const R* __restrict__ tacc,
                                          const R* __restrict__ fv, int i, int j, int k,
                                          long long id, R r[5]) {
     cell_visc<R, ORD>(P, fv, i, j, k, id, r);
-    const long long n = P.n;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) r[q] += -tacc[q * n + id];
+    for (int q = 0; q < 5; ++q) r[q] += -acc_term<R, T3>(P, tacc, q, id);
 }
 
 // compute_rhs output (5 blocks of n, double).
-template <class R, int ORD>
+template <class R, int ORD, bool T3>
 __global__ void __launch_bounds__(128)
 k_rhs_out(DevParams P, const R* __restrict__ tacc, const R* __restrict__ fv,
           double* __restrict__ rhs) {
@@ -1234,7 +1249,7 @@ k_rhs_out(DevParams P, const R* __restrict__ tacc, const R* __restrict__ fv,
     const int j = blockIdx.y, k = blockIdx.z;
     const long long id = ((long long)k * P.ny + j) * P.nx + i;
     R r[5];
-    cell_rhs<R, ORD>(P, tacc, fv, i, j, k, id, r);
+    cell_rhs<R, ORD, T3>(P, tacc, fv, i, j, k, id, r);
 #pragma unroll
     for (int q = 0; q < 5; ++q) rhs[q * P.n + id] = double(r[q]);
 }
@@ -1402,7 +1417,7 @@ __device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& 
 // are latency-bound, and more resident warps beat more loads in flight per
 // thread. Measured at 256^3: FP32 0.713 -> 0.578 ms (5 blocks 0.630, 7 blocks
 // 0.609, 10 blocks 0.680); FP64 1.80 -> 1.39 ms (6 blocks 1.52, 10 blocks 1.55).
-template <class R, int ORD, int STAGE>
+template <class R, int ORD, int STAGE, bool T3>
 __global__ void __launch_bounds__(128, 8)
 k_update(DevParams P, StateView Wc, StateView W0, const R* __restrict__ tacc,
          const R* __restrict__ fv, StateOut Wn, Ctrl* ctrl) {
@@ -1414,7 +1429,7 @@ k_update(DevParams P, StateView Wc, StateView W0, const R* __restrict__ tacc,
     double cand = CFL_INIT;
     if (live) {
         R r[5];
-        cell_rhs<R, ORD>(P, tacc, fv, i, j, k, id, r);
+        cell_rhs<R, ORD, T3>(P, tacc, fv, i, j, k, id, r);
         stage_cell<R, STAGE>(P, Wc, W0, id, r, ctrl->dt, Wn, ctrl, cand);
     }
     if (STAGE == 3) block_min_to(cand, &ctrl->dtmin_bits);

@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "ns3d_kernels.cuh"
+#include "ns3d_small.cuh"
 
 namespace ns3d {
 
@@ -20,6 +21,7 @@ struct LaunchCfg {
     cudaStream_t stream;
     int zb;       // planes per block of the 2.5-D viscous kernels (0: from the grid)
     int tiled;    // bit 0: 2.5-D visc_flux (when the box tiles); bit 1: its pipelined form
+    long long small;  // FP64 boxes of at most so many cells take k_flux_small (see small_box)
     int pipe;     // FP32 sweeps with the software-pipelined split: bit 0 the x sweep
                   // (k_sweep_x_pipe, rows of >= 128 cells), bit 1 the y / z sweeps (k_sweep_pipe)
 };
@@ -33,11 +35,15 @@ template <class R>
 cudaError_t launch_sweep(const LaunchCfg& L, int dir, StateView W, R* tacc, const Ctrl* ctrl);
 template <class R>
 cudaError_t launch_visc_flux(const LaunchCfg& L, StateView W, R* fv, const Ctrl* ctrl);
+// t3: T_acc as the three separate terms of launch_flux_small.
 template <class R>
 cudaError_t launch_update(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
-                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl);
+                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl, bool t3);
 template <class R>
-cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs);
+cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs, bool t3);
+// All fluxes of an FP64 right-hand side in one launch (k_flux_small): tacc (15
+// blocks of n) and fv. For boxes of small_box() only.
+cudaError_t launch_flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl);
 // The z sweep fused with the stage update (k_sweep_ring<2, ..., FUSE>): T_acc
 // holds the x + y terms, fv the viscous fluxes of Wc; writes Wn. Component-wise
 // reconstruction only (L.chr == 0; cudaErrorNotSupported otherwise).
@@ -62,6 +68,14 @@ inline int segment_for(int len, long long lines) {
 }
 
 }  // namespace detail
+
+// Whether an FP64 box takes launch_flux_small: component-wise schemes, few
+// enough cells, every line short enough for a block's shared memory, no tuning
+// override of the marching kernels.
+inline bool small_box(const LaunchCfg& L) {
+    const DevParams& P = L.P;
+    return L.small && !L.chr && P.n <= L.small && P.nx <= SMALL_NC && P.ny <= SMALL_NC && P.nz <= SMALL_NC;
+}
 
 #ifdef NS3D_LAUNCH_IMPL
 
@@ -265,45 +279,115 @@ cudaError_t launch_visc_flux(const LaunchCfg& L, StateView W, R* fv, const Ctrl*
     return cudaGetLastError();
 }
 
-template <class R, int ORD>
+template <class R, int ORD, bool T3>
 static cudaError_t update_ord(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
                               const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl) {
     const int th = detail::threads_for(L.P.nx);
     const dim3 g = detail::cell_grid(L.P, th);
-    if (stage == 1) k_update<R, ORD, 1><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
-    else if (stage == 2) k_update<R, ORD, 2><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
-    else k_update<R, ORD, 3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
+    if (stage == 1) k_update<R, ORD, 1, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
+    else if (stage == 2) k_update<R, ORD, 2, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
+    else k_update<R, ORD, 3, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
     return cudaGetLastError();
+}
+
+// f(std::bool_constant<T3>): the separate terms exist in the FP64 form only.
+template <class R, class F>
+cudaError_t by_terms(bool t3, F f) {
+    if constexpr (sizeof(R) == 8) {
+        if (t3) return f(std::true_type{});
+    }
+    return f(std::false_type{});
 }
 
 template <class R>
 cudaError_t launch_update(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
-                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl) {
-    switch (L.P.vis_order) {
-    case 4: return update_ord<R, 4>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-    case 6: return update_ord<R, 6>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-    default: return update_ord<R, 8>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-    }
+                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl, bool t3) {
+    return by_terms<R>(t3, [&](auto t) -> cudaError_t {
+        constexpr bool T3 = decltype(t)::value;
+        switch (L.P.vis_order) {
+        case 4: return update_ord<R, 4, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+        case 6: return update_ord<R, 6, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+        default: return update_ord<R, 8, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+        }
+    });
 }
 
 template <class R>
-cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs) {
+cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs, bool t3) {
     const int th = detail::threads_for(L.P.nx);
     const dim3 g = detail::cell_grid(L.P, th);
-    switch (L.P.vis_order) {
-    case 4: k_rhs_out<R, 4><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
-    case 6: k_rhs_out<R, 6><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
-    default: k_rhs_out<R, 8><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+    return by_terms<R>(t3, [&](auto t) -> cudaError_t {
+        constexpr bool T3 = decltype(t)::value;
+        switch (L.P.vis_order) {
+        case 4: k_rhs_out<R, 4, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+        case 6: k_rhs_out<R, 6, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+        default: k_rhs_out<R, 8, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+        }
+        return cudaGetLastError();
+    });
+}
+
+#ifdef NS3D_LAUNCH_SMALL
+namespace detail {
+inline SmallShape small_shape(const LaunchCfg& L) {
+    const DevParams& P = L.P;
+    SmallShape sh{};
+    // lines per block: 64 to 256 cells, so that the three sweeps give at least
+    // two blocks per SM; four lines or more along y and z (32-byte rows)
+    long long target = 3 * P.n / (2 * 148);
+    target = target < 64 ? 64 : (target > 256 ? 256 : target);
+    for (int d = 0; d < 3; ++d) {
+        const int len = d == 0 ? P.nx : (d == 1 ? P.ny : P.nz);
+        const long long lines = d == 0 ? (long long)P.ny * P.nz : P.nx;
+        long long lb = (target + len / 2) / len;
+        if (d > 0 && lb < 4) lb = 4;
+        if (lb > SMALL_NC / len) lb = SMALL_NC / len;
+        if (lb > lines) lb = lines;
+        if (lb < 1) lb = 1;
+        sh.lb[d] = (int)lb;
+        sh.nb[d] = (int)((lines + lb - 1) / lb) * (d == 0 ? 1 : (d == 1 ? P.nz : P.ny));
     }
+    sh.nb[3] = (int)((P.n + SMALL_T - 1) / SMALL_T);
+    return sh;
+}
+
+template <int FVS, int RC>
+cudaError_t flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
+    const SmallShape sh = small_shape(L);
+    int nc = 0;
+    for (int d = 0; d < 3; ++d) {
+        const int c = sh.lb[d] * (d == 0 ? L.P.nx : (d == 1 ? L.P.ny : L.P.nz));
+        nc = c > nc ? c : nc;
+    }
+    const unsigned blocks = (unsigned)(sh.nb[0] + sh.nb[1] + sh.nb[2] + sh.nb[3]);
+    k_flux_small<FVS, RC><<<blocks, SMALL_T, small_smem(nc), L.stream>>>(L.P, W, tacc, fv, sh, ctrl);
     return cudaGetLastError();
 }
+}  // namespace detail
+
+cudaError_t launch_flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
+    auto by_rc = [&](auto fvs) -> cudaError_t {
+        constexpr int FVS = decltype(fvs)::value;
+        switch (L.rc) {
+        case RC_WENO5: return detail::flux_small<FVS, RC_WENO5>(L, W, tacc, fv, ctrl);
+        case RC_LINEAR: return detail::flux_small<FVS, RC_LINEAR>(L, W, tacc, fv, ctrl);
+        case RC_LIN6: return detail::flux_small<FVS, RC_LIN6>(L, W, tacc, fv, ctrl);
+        case RC_MDCD_HYBRID: return detail::flux_small<FVS, RC_MDCD_HYBRID>(L, W, tacc, fv, ctrl);
+        case RC_LIN8: return detail::flux_small<FVS, RC_LIN8>(L, W, tacc, fv, ctrl);
+        default: return cudaErrorInvalidValue;
+        }
+    };
+    return L.fvs == FV_SW ? by_rc(std::integral_constant<int, FV_SW>{})
+                          : by_rc(std::integral_constant<int, FV_LF>{});
+}
+#endif  // NS3D_LAUNCH_SMALL
 
 #define NS3D_INSTANTIATE_LAUNCHERS(R)                                                          \
     template cudaError_t launch_sweep<R>(const LaunchCfg&, int, StateView, R*, const Ctrl*);   \
     template cudaError_t launch_visc_flux<R>(const LaunchCfg&, StateView, R*, const Ctrl*);    \
     template cudaError_t launch_update<R>(const LaunchCfg&, int, StateView, StateView,         \
-                                          const R*, const R*, StateOut, Ctrl*);                \
-    template cudaError_t launch_rhs_out<R>(const LaunchCfg&, const R*, const R*, double*);   \
+                                          const R*, const R*, StateOut, Ctrl*, bool);          \
+    template cudaError_t launch_rhs_out<R>(const LaunchCfg&, const R*, const R*, double*, bool); \
     template cudaError_t launch_sweep_z_update<R>(const LaunchCfg&, int, StateView, StateView, \
                                                   const R*, const R*, StateOut, Ctrl*);
 

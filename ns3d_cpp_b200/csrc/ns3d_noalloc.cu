@@ -31,10 +31,10 @@ using namespace ns3d;
 namespace ns3d {
 extern template cudaError_t launch_sweep<double>(const LaunchCfg&, int, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<double>(const LaunchCfg&, StateView, double*, const Ctrl*);
-extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*);
+extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*, bool);
 extern template cudaError_t launch_sweep<float>(const LaunchCfg&, int, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<float>(const LaunchCfg&, StateView, float*, const Ctrl*);
-extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*);
+extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*, bool);
 }  // namespace ns3d
 
 // 15 doubles per cell: T (double) + 5 accumulator values + the viscous fluxes
@@ -88,13 +88,21 @@ template <class R>
 cudaError_t rhs_into(const LaunchCfg& L, StateView W, double* scratch, double* rhs) {
     const long long n = L.P.n;
     R* tacc = reinterpret_cast<R*>(scratch + n);
+    // FP64: the one-launch flux kernel keeps the three directions' terms apart,
+    // (1 + 15 + 9) doubles per cell, which the scratch holds up to 39321 cells
+    const bool t3 = sizeof(R) == 8 && small_box(L) && 25 * n <= 15 * (long long)NS3D_NOALLOC_MAX_CELLS;
     // fv on a 16-byte boundary (the FP32 form reads it as float4); FP32 needs
     // 8 + 20 + 48 bytes per cell (+12 of padding) of the 120 the array holds
-    R* fv = reinterpret_cast<R*>((reinterpret_cast<uintptr_t>(tacc + 5 * n) + 15) & ~uintptr_t(15));
+    R* fv = reinterpret_cast<R*>((reinterpret_cast<uintptr_t>(tacc + (t3 ? 15 : 5) * n) + 15) & ~uintptr_t(15));
     cudaError_t e = cudaSuccess;
-    for (int dir = 0; dir < 3 && e == cudaSuccess; ++dir) e = launch_sweep<R>(L, dir, W, tacc, nullptr);
-    if (e == cudaSuccess) e = launch_visc_flux<R>(L, W, fv, nullptr);
-    if (e == cudaSuccess) e = launch_rhs_out<R>(L, tacc, fv, rhs);
+    if constexpr (sizeof(R) == 8) {
+        if (t3) e = launch_flux_small(L, W, tacc, fv, nullptr);
+    }
+    if (!t3) {
+        for (int dir = 0; dir < 3 && e == cudaSuccess; ++dir) e = launch_sweep<R>(L, dir, W, tacc, nullptr);
+        if (e == cudaSuccess) e = launch_visc_flux<R>(L, W, fv, nullptr);
+    }
+    if (e == cudaSuccess) e = launch_rhs_out<R>(L, tacc, fv, rhs, t3);
     return e;
 }
 

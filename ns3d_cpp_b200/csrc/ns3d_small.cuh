@@ -1,0 +1,147 @@
+// The flux part of one FP64 right-hand side in one launch: the x, y and z
+// sweeps and the viscous flux run side by side as blocks of different roles.
+//
+// On a small box the marching sweeps are bound by latency, not by any pipe:
+// one thread splits S cells and reconstructs its faces one after the other, the
+// launches depend on each other through T_acc, and a 32^3 box has 1024 lines
+// for 148 SMs. Here a block takes a few whole periodic lines into shared
+// memory: every thread splits one cell, then reconstructs one component of one
+// face (five times the parallelism, no halo cells, no serial march), then
+// differences. Each direction writes its own term, so nothing depends on
+// another launch; the reader adds them in T_acc's order (acc_term). The
+// operations per cell and face are those of the marching kernels: same bits.
+//
+// FP64 only: the FP32 form's reconstructions work on float deviations from an
+// offset per marching segment, and its roundings belong to the marching kernels.
+#pragma once
+
+#include "ns3d_kernels.cuh"
+
+namespace ns3d {
+
+#ifndef NS3D_SMALL_T
+#define NS3D_SMALL_T 128
+#endif
+constexpr int SMALL_T = NS3D_SMALL_T;  // threads per block
+constexpr int SMALL_NC = 400;          // cells of a block's lines, at most (48 KB of shared memory)
+
+// Launch shape: blocks per role (x, y, z, viscous), lines per block.
+struct SmallShape {
+    int nb[4], lb[3];
+};
+
+constexpr int small_smem(int nc) { return nc * 15 * (int)sizeof(double); }
+
+// The sweep along DIR of the lines of block b: out (5 blocks of n).
+template <int DIR, int FVS, int RC>
+__device__ __forceinline__ void small_sweep(const DevParams& P, const StateView& W,
+                                            double* __restrict__ out, int b, int lb, double* sm) {
+    constexpr int S = Stencil<RC>::S;
+    constexpr int MID = (S - 1) / 2;
+    const int nx = P.nx, ny = P.ny, nz = P.nz;
+    const long long n = P.n;
+    const int len = DIR == 0 ? nx : (DIR == 1 ? ny : nz);
+    // line l of the block, position s: cell id0 + l dl + s ds, slot l cl + s cs
+    long long id0, dl, ds;
+    int nl;
+    if constexpr (DIR == 0) {
+        const int l0 = b * lb;
+        nl = min(lb, ny * nz - l0);
+        id0 = (long long)l0 * nx; dl = nx; ds = 1;
+    } else {
+        const int gx = (nx + lb - 1) / lb, o = b / gx, i0 = (b - o * gx) * lb;
+        nl = min(lb, nx - i0);
+        id0 = (DIR == 1 ? (long long)o * ny : (long long)o) * nx + i0;
+        dl = 1;
+        ds = DIR == 1 ? (long long)nx : (long long)nx * ny;
+    }
+    const int cl = DIR == 0 ? len : 1, cs = DIR == 0 ? 1 : nl;
+    const int nc = nl * len;
+    double* F = sm;             // [10][nc]: F+0..4, F-0..4
+    double* fl = sm + 10 * nc;  // [5][nc]: face right of each cell
+    auto line_of_slot = [&](int c, int& l, int& s) {
+        if constexpr (DIR == 0) { l = c / len; s = c - l * len; }
+        else { s = c / nl; l = c - s * nl; }
+    };
+    for (int c = threadIdx.x; c < nc; c += SMALL_T) {
+        int l, s;
+        line_of_slot(c, l, s);
+        const long long id = id0 + l * dl + s * ds;
+        const double raw[5] = {W.rho[id], W.u[id], W.v[id], W.w[id], W.p[id]};
+        double Fp[5], Fm[5];
+        split_fp64<FVS, RC, DIR == 0, DIR == 1, DIR == 2>(P, raw, Fp, Fm);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            F[q * nc + c] = Fp[q];
+            F[(5 + q) * nc + c] = Fm[q];
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 5 * nc; t += SMALL_T) {
+        // component q of the face between positions s and s+1 of line l
+        const int q = t / nc, c = t - q * nc;
+        int l, s;
+        line_of_slot(c, l, s);
+        const double* fp = F + q * nc + l * cl;
+        const double* fm = fp + 5 * nc;
+        double a[S], bm[S];
+#pragma unroll
+        for (int m = 0; m < S; ++m) {
+            const int w = wrap1(s - MID + m, len) * cs;
+            a[m] = fp[w];
+            bm[S - 1 - m] = fm[w];  // reconstruct_select reverses for flag < 0
+        }
+        double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
+                   reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
+        if constexpr (RC == RC_WENO5) {  // as in recon_face
+            if (!finite_hi(f))
+                f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
+                    weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
+        }
+        fl[t] = f;
+    }
+    __syncthreads();
+    const double inv_h = DIR == 0 ? P.inv_dx : (DIR == 1 ? P.inv_dy : P.inv_dz);
+    for (int t = threadIdx.x; t < 5 * nc; t += SMALL_T) {
+        const int q = t / nc, c = t - q * nc;
+        int l, s;
+        line_of_slot(c, l, s);
+        const double d = fl[t] - fl[q * nc + l * cl + wrap1(s - 1, len) * cs];
+        out[q * n + id0 + l * dl + s * ds] = d * inv_h;
+    }
+}
+
+// t3: 15 blocks of n, the x, y and z terms of the five components; fv: the
+// viscous fluxes in store_fv's layout.
+template <int FVS, int RC>
+__global__ void __launch_bounds__(SMALL_T, 512 / SMALL_T)
+k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restrict__ fv, SmallShape sh,
+             const Ctrl* __restrict__ ctrl) {
+    if (ctrl && ctrl->stop) return;
+    extern __shared__ double small_sm[];
+    const long long n = P.n;
+    int b = blockIdx.x;
+    if (b < sh.nb[0]) {
+        small_sweep<0, FVS, RC>(P, W, t3, b, sh.lb[0], small_sm);
+        return;
+    }
+    b -= sh.nb[0];
+    if (b < sh.nb[1]) {
+        small_sweep<1, FVS, RC>(P, W, t3 + 5 * n, b, sh.lb[1], small_sm);
+        return;
+    }
+    b -= sh.nb[1];
+    if (b < sh.nb[2]) {
+        small_sweep<2, FVS, RC>(P, W, t3 + 10 * n, b, sh.lb[2], small_sm);
+        return;
+    }
+    b -= sh.nb[2];
+    const int c = b * SMALL_T + threadIdx.x;
+    if (c >= n) return;
+    const int i = c % P.nx, jk = c / P.nx, j = jk % P.ny, k = jk / P.ny;
+    if (P.vis_order == 4) visc_cell<double, 4>(P, W, fv, i, j, k);
+    else if (P.vis_order == 6) visc_cell<double, 6>(P, W, fv, i, j, k);
+    else visc_cell<double, 8>(P, W, fv, i, j, k);
+}
+
+}  // namespace ns3d
