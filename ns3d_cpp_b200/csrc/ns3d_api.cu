@@ -28,13 +28,13 @@ namespace ns3d {
 extern template cudaError_t launch_sweep<double>(const LaunchCfg&, int, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<double>(const LaunchCfg&, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_update<double>(const LaunchCfg&, int, StateView, StateView,
-                                                  const double*, const double*, StateOut, Ctrl*, bool);
-extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*, bool);
+                                                  const double*, const double*, StateOut, Ctrl*);
+extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*);
 extern template cudaError_t launch_sweep<float>(const LaunchCfg&, int, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<float>(const LaunchCfg&, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_update<float>(const LaunchCfg&, int, StateView, StateView,
-                                                 const float*, const float*, StateOut, Ctrl*, bool);
-extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*, bool);
+                                                 const float*, const float*, StateOut, Ctrl*);
+extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*);
 extern template cudaError_t launch_sweep_z_update<double>(const LaunchCfg&, int, StateView, StateView,
                                                           const double*, const double*, StateOut, Ctrl*);
 extern template cudaError_t launch_sweep_z_update<float>(const LaunchCfg&, int, StateView, StateView,
@@ -583,8 +583,15 @@ ns3d_status stage_t(ns3d_ctx* ctx, int stage, StateView Wc, StateView W0, StateO
     if (ctx->L.chr || !ctx->fuse) {
         ns3d_status s = rhs_parts_t<R>(ctx, Wc, ctx->ctrl);
         if (s != NS3D_OK) return s;
+        if constexpr (sizeof(R) == 8) {
+            if (ctx->t3) {
+                NS3D_LAUNCH(NS3D_KERNEL_UPDATE, 1, launch_update_small(ctx->L, stage, Wc, W0, tacc, fv, Wn,
+                                                                       ctx->ctrl, nullptr));
+                return NS3D_OK;
+            }
+        }
         NS3D_LAUNCH(NS3D_KERNEL_UPDATE, 1,
-                    launch_update<R>(ctx->L, stage, Wc, W0, tacc, fv, Wn, ctx->ctrl, ctx->t3));
+                    launch_update<R>(ctx->L, stage, Wc, W0, tacc, fv, Wn, ctx->ctrl));
         return NS3D_OK;
     }
     ns3d_status s = rhs_parts_t<R>(ctx, Wc, ctx->ctrl, 2);
@@ -749,6 +756,8 @@ void default_tiling(LaunchCfg& L) {
     L.pipe = 3;   // FP32 sweeps with the software-pipelined split (k_sweep_x_pipe, k_sweep_pipe)
     // an override of the marching kernels' shapes selects those kernels
     L.small = 300000;
+    L.pdl = 1;  // where pdl_box() holds
+    if (const char* e = std::getenv("NS3D_PDL")) L.pdl = std::atoi(e);
     for (const char* v : {"NS3D_TILE_ZB", "NS3D_TILED", "NS3D_SEG"})
         if (std::getenv(v)) L.small = 0;
     if (const char* e = std::getenv("NS3D_SMALL")) L.small = std::atoll(e);
@@ -836,6 +845,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     ctx->L.chr = q.char_recon ? 1 : 0;
     for (int d = 0; d < 3; ++d) ctx->L.seg[d] = 0;  // chosen per launch from the grid
     default_tiling(ctx->L);
+    if (!pdl_box(P, q.precision == NS3D_PREC_FP64)) ctx->L.pdl = 0;
     ctx->rsize = q.precision == NS3D_PREC_FP64 ? sizeof(double) : sizeof(float);
 
     auto bail = [&](ns3d_status st, const std::string& m) {
@@ -850,6 +860,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     ctx->L.stream = ctx->stream;
     if (const char* ov = std::getenv("NS3D_OVERLAP")) ctx->overlap = std::atoi(ov) != 0;
     if (const char* fu = std::getenv("NS3D_FUSE")) ctx->fuse = std::atoi(fu) != 0;
+    if (ctx->overlap) ctx->L.pdl = 0;  // kernels of two streams depend on each other
     if (ctx->overlap &&
         (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
          cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -1065,12 +1076,16 @@ ns3d_status ns3d_compute_rhs(ns3d_ctx* ctx, double* r0, double* r1, double* r2, 
     // rhs staged in a free state buffer (5 of its 6 arrays)
     const int tmpb = ctx->cur == ctx->rec ? (ctx->cur + 1) % 3 : 3 - ctx->cur - ctx->rec;
     double* rhs = warr(ctx, tmpb, 0);
-    if (ctx->p.precision == NS3D_PREC_FP64)
+    if (ctx->t3)
         NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    launch_rhs_out<double>(ctx->L, (const double*)ctx->tacc, (const double*)ctx->fv, rhs, ctx->t3));
+                    launch_update_small(ctx->L, 0, StateView{}, StateView{}, (const double*)ctx->tacc,
+                                        (const double*)ctx->fv, StateOut{}, nullptr, rhs));
+    else if (ctx->p.precision == NS3D_PREC_FP64)
+        NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
+                    launch_rhs_out<double>(ctx->L, (const double*)ctx->tacc, (const double*)ctx->fv, rhs));
     else
         NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    launch_rhs_out<float>(ctx->L, (const float*)ctx->tacc, (const float*)ctx->fv, rhs, ctx->t3));
+                    launch_rhs_out<float>(ctx->L, (const float*)ctx->tacc, (const float*)ctx->fv, rhs));
     const double* d[5];
     for (int q = 0; q < 5; ++q) d[q] = rhs + q * ctx->n;
     double* h[5] = {r0, r1, r2, r3, r4};
@@ -1142,15 +1157,17 @@ static ns3d_status run_steps(ns3d_ctx* ctx, int mode, int nsteps, int* steps_don
         return s;
     const ns3d_params& p = ctx->p;
     const int cur0 = ctx->cur, rec0 = ctx->rec;
+    auto control = [&](int what) -> ns3d_status {
+        NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
+                    launch_pdl(ctx->L, k_control, 1, 1, 0, ctx->ctrl, what, mode, p.cfl, p.dt_fixed, p.TotalTime,
+                               p.output_Timefreq, ctx->n, ctx->step_times));
+        return NS3D_OK;
+    };
+    if (nsteps > 0 && (s = control(CONTROL_PRE)) != NS3D_OK) return s;
     for (int step = 0; step < nsteps; ++step) {
         ctx->rec = ctx->cur;  // recordConservedTo0 (maincycle.cpp:22)
-        NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    (k_control_pre<<<1, 1, 0, ctx->stream>>>(ctx->ctrl, mode, p.cfl, p.dt_fixed,
-                                                              p.TotalTime, p.output_Timefreq)));
         if ((s = enqueue_rk3(ctx)) != NS3D_OK) return s;
-        NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                    (k_control_post<<<1, 1, 0, ctx->stream>>>(ctx->ctrl, mode, p.TotalTime, ctx->n,
-                                                               ctx->step_times)));
+        if ((s = control(step + 1 < nsteps ? CONTROL_POST | CONTROL_PRE : CONTROL_POST)) != NS3D_OK) return s;
     }
     if ((s = read_ctrl(ctx)) != NS3D_OK) return s;
     const Ctrl& h = *ctx->ctrl_host;
@@ -1595,8 +1612,8 @@ ns3d_status ns3d_adjoint(ns3d_ctx* ctx, int nsteps, int K, const double* dts_in,
                                     sizeof(unsigned long long), cudaMemcpyHostToDevice, ctx->stream));
             if ((s = enqueue_cfl(ctx)) != NS3D_OK) return s;
             NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
-                        (k_control_pre<<<1, 1, 0, ctx->stream>>>(ctx->ctrl, 0, ctx->p.cfl,
-                                                                  ctx->p.dt_fixed, 0.0, 0.0)));
+                        launch_pdl(ctx->L, k_control, 1, 1, 0, ctx->ctrl, (int)CONTROL_PRE, 0, ctx->p.cfl,
+                                   ctx->p.dt_fixed, 0.0, 0.0, n, (double*)nullptr));
         }
         NS3D_CK(cudaMemcpyAsync(dtd + k, &ctx->ctrl->dt, sizeof(double), cudaMemcpyDeviceToDevice,
                                 ctx->stream));

@@ -55,6 +55,18 @@ __device__ __forceinline__ int wrap1(int s, int len) {
     return s < 0 ? s + len : (s >= len ? s - len : s);
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute may start
+// while its predecessor drains; pdl_wait returns when all that precedes it is
+// complete and visible (at once in a plain launch), pdl_trigger lets the
+// successor's launch begin (it waits in turn). Every kernel launched with the
+// attribute waits before its first read or write of device memory.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+    pdl_wait();
+    pdl_trigger();
+}
+
 // ---------------------------------------------------------------------------
 // One face of du_inviscous_character (InviscousFlux_new.cpp:165-437): the Roe
 // state of the face's two cells wl, wr (primitives, rho as stored), the
@@ -212,6 +224,7 @@ __device__ __forceinline__ void ring_window_at(int ph, const SplitRing<R, S, T>&
 template <int DIR, class R, int FVS, int RC, bool CHR = false>
 __global__ void __launch_bounds__(128)
 k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
@@ -382,6 +395,7 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
 template <class R, int FVS, int RC, bool CHR = false>
 __global__ void __launch_bounds__(32 * XW_WARPS)
 k_sweep_x_warp(DevParams P, StateView W, R* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     __shared__ SplitRing<R, XW_WARPS, 96> ring;  // [warp][3 chunks x 32 cells]
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
@@ -397,6 +411,7 @@ k_sweep_x_warp(DevParams P, StateView W, R* __restrict__ tacc, const Ctrl* __res
 template <int FVS, int RC>
 __global__ void __maxnreg__(128)
 k_sweep_x_warp_f32(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     __shared__ SplitRing<float, XW_WARPS, 96> ring;
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
@@ -418,6 +433,7 @@ k_sweep_x_warp_f32(DevParams P, StateView W, float* __restrict__ tacc, const Ctr
 template <int FVS, int RC, int ENT>
 __global__ void __launch_bounds__(32 * XW_WARPS, 4)
 k_sweep_x_pipe(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
@@ -823,6 +839,7 @@ __device__ __forceinline__ void visc_cell(const DevParams& P, const StateView& W
 template <class R, int ORD>
 __global__ void __launch_bounds__(128)
 k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.nx) return;
@@ -853,6 +870,7 @@ k_visc_flux_25d(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __rest
                 int zb) {
     constexpr int VT_X = VTile<R>::X, VT_Y = VTile<R>::Y, VT_H = VTile<R>::H;
     constexpr int VT_SX = VTile<R>::SX, VT_SY = VTile<R>::SY;
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     // FP32-stencil form: values enter the tile and the z queue as float
     // deviations from one reference per block and variable (formed in
@@ -1000,6 +1018,7 @@ k_visc_flux_pipe(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __res
     using VP = VPipe<R>;
     constexpr int X = VT::X, Y = VT::Y, H = VT::H, SX = VT::SX, SY = VT::SY;
     constexpr int NT = VP::NT, NH = VP::NH, HPT = VP::HPT;
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     constexpr bool kDeviation = sizeof(R) < sizeof(double);
     extern __shared__ __align__(16) unsigned char vsm[];
@@ -1221,26 +1240,26 @@ __device__ __forceinline__ void cell_visc(const DevParams& P, const R* __restric
 // T_acc of one cell and component. T3 (FP64 form): from the separate x, y and
 // z terms of k_flux_small (15 blocks of n), added in the marching sweeps' order.
 template <class R, bool T3>
-__device__ __forceinline__ R acc_term(const DevParams& P, const R* __restrict__ tacc, int q, long long id) {
+__device__ __forceinline__ R acc_term(const R* __restrict__ tacc, long long n, int q, long long id) {
     static_assert(!T3 || sizeof(R) == 8, "separate terms belong to the FP64 form");
-    const long long n = P.n;
     if constexpr (T3) return (tacc[q * n + id] + tacc[(5 + q) * n + id]) + tacc[(10 + q) * n + id];
     else return tacc[q * n + id];
 }
 
 // rhs at one cell: the viscous part followed by the inviscid divergence
 // (range_kutta.cpp:61-97) accumulated in tacc.
-template <class R, int ORD, bool T3>
+template <class R, int ORD, bool T3 = false>
 __device__ __forceinline__ void cell_rhs(const DevParams& P, const R* __restrict__ tacc,
                                          const R* __restrict__ fv, int i, int j, int k,
                                          long long id, R r[5]) {
     cell_visc<R, ORD>(P, fv, i, j, k, id, r);
+    const long long n = P.n;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) r[q] += -acc_term<R, T3>(P, tacc, q, id);
+    for (int q = 0; q < 5; ++q) r[q] += -acc_term<R, T3>(tacc, n, q, id);
 }
 
 // compute_rhs output (5 blocks of n, double).
-template <class R, int ORD, bool T3>
+template <class R, int ORD>
 __global__ void __launch_bounds__(128)
 k_rhs_out(DevParams P, const R* __restrict__ tacc, const R* __restrict__ fv,
           double* __restrict__ rhs) {
@@ -1249,7 +1268,7 @@ k_rhs_out(DevParams P, const R* __restrict__ tacc, const R* __restrict__ fv,
     const int j = blockIdx.y, k = blockIdx.z;
     const long long id = ((long long)k * P.ny + j) * P.nx + i;
     R r[5];
-    cell_rhs<R, ORD, T3>(P, tacc, fv, i, j, k, id, r);
+    cell_rhs<R, ORD>(P, tacc, fv, i, j, k, id, r);
 #pragma unroll
     for (int q = 0; q < 5; ++q) rhs[q * P.n + id] = double(r[q]);
 }
@@ -1332,15 +1351,13 @@ __device__ __forceinline__ void prim2cons_fast(const StateView& W, long long id,
 
 // Shu-Osher stage of one cell from its rhs r, conservedToPrimitive of the
 // result and, after stage 3, the positivity test and the CFL candidate
-// (folded into `cand` with std::min semantics: a NaN never wins).
+// (folded into `cand` with std::min semantics: a NaN never wins). stage_load:
+// the recorded and (stages 2, 3) the current conserved state.
 template <class R, int STAGE>
-__device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& Wc,
-                                           const StateView& W0, long long id, const R r[5],
-                                           double dt, const StateOut& Wn, Ctrl* ctrl,
-                                           double& cand) {
+__device__ __forceinline__ void stage_load(const DevParams& P, const StateView& Wc, const StateView& W0,
+                                           long long id, double U0[5], double U[5]) {
     constexpr bool kFast = sizeof(R) < sizeof(double);
     const double gamma = P.gamma;
-    double U0[5], U[5];
     if constexpr (kFast) {
         const double inv_gm1 = 1.0 / (gamma - 1.0);
         prim2cons_fast(W0, id, inv_gm1, U0);
@@ -1349,6 +1366,14 @@ __device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& 
         prim2cons_cell(W0, id, gamma, U0);
         if (STAGE != 1) prim2cons_cell(Wc, id, gamma, U);
     }
+}
+
+template <class R, int STAGE>
+__device__ __forceinline__ void stage_apply(const DevParams& P, const double U0[5], double U[5],
+                                            long long id, const R r[5], double dt, const StateOut& Wn,
+                                            Ctrl* ctrl, double& cand) {
+    constexpr bool kFast = sizeof(R) < sizeof(double);
+    const double gamma = P.gamma;
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         const double rq = double(r[q]);
@@ -1413,14 +1438,25 @@ __device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& 
     }
 }
 
+template <class R, int STAGE>
+__device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& Wc,
+                                           const StateView& W0, long long id, const R r[5],
+                                           double dt, const StateOut& Wn, Ctrl* ctrl,
+                                           double& cand) {
+    double U0[5], U[5];
+    stage_load<R, STAGE>(P, Wc, W0, id, U0, U);
+    stage_apply<R, STAGE>(P, U0, U, id, r, dt, Wn, ctrl, cand);
+}
+
 // 8 blocks of 128 threads per SM (at most 64 registers): the neighbour loads
 // are latency-bound, and more resident warps beat more loads in flight per
 // thread. Measured at 256^3: FP32 0.713 -> 0.578 ms (5 blocks 0.630, 7 blocks
 // 0.609, 10 blocks 0.680); FP64 1.80 -> 1.39 ms (6 blocks 1.52, 10 blocks 1.55).
-template <class R, int ORD, int STAGE, bool T3>
+template <class R, int ORD, int STAGE, bool T3 = false>
 __global__ void __launch_bounds__(128, 8)
 k_update(DevParams P, StateView Wc, StateView W0, const R* __restrict__ tacc,
          const R* __restrict__ fv, StateOut Wn, Ctrl* ctrl) {
+    pdl_enter();
     if (ctrl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < P.nx;
@@ -1496,6 +1532,7 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     constexpr int T = RingCfg<R>::T;
     constexpr bool kDeviation = sizeof(R) < sizeof(double);
     __shared__ SplitRing<R, S, T> ring;
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long n = P.n;
@@ -1642,6 +1679,7 @@ k_sweep_pipe(DevParams P, StateView W, float* __restrict__ tacc, int seg,
     constexpr int MID = (S - 1) / 2;
     constexpr int T = RingCfg<float>::T;
     __shared__ SplitRing<float, S, T> ring;
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long n = P.n;
@@ -1777,8 +1815,8 @@ k_cfl(DevParams P, StateView W, Ctrl* ctrl) {
 // clipping and stop conditions of time_advance; mode 2: as mode 1, and the
 // loop also ends after a step whose if_output is set, so that the host can
 // write that step's output.
-__global__ void k_control_pre(Ctrl* c, int mode, double cfl, double dt_fixed, double total_time,
-                              double out_freq) {
+__device__ void control_pre(Ctrl* c, int mode, double cfl, double dt_fixed, double total_time,
+                            double out_freq) {
     if (c->stop) return;
     const double eps = 1e-12;
     c->output = 0;
@@ -1820,8 +1858,7 @@ __global__ void k_control_pre(Ctrl* c, int mode, double cfl, double dt_fixed, do
 }
 
 // End of one iteration (maincycle.cpp:250 + 298-300, range_kutta.cpp:149-162).
-__global__ void k_control_post(Ctrl* c, int mode, double total_time, long long n,
-                               double* times) {
+__device__ void control_post(Ctrl* c, int mode, double total_time, long long n, double* times) {
     if (c->stop || !c->active) return;
     c->active = 0;
     c->steps_done += 1;
@@ -1838,6 +1875,16 @@ __global__ void k_control_post(Ctrl* c, int mode, double total_time, long long n
         c->stop = 1;
         c->stop_reason = STOP_OUTPUT;
     }
+}
+
+// The loop's control between two steps in one launch: the end of the step that
+// ran (POST) and the start of the next one (PRE).
+enum : int { CONTROL_POST = 1, CONTROL_PRE = 2 };
+__global__ void k_control(Ctrl* c, int what, int mode, double cfl, double dt_fixed, double total_time,
+                          double out_freq, long long n, double* times) {
+    pdl_enter();
+    if (what & CONTROL_POST) control_post(c, mode, total_time, n, times);
+    if (what & CONTROL_PRE) control_pre(c, mode, cfl, dt_fixed, total_time, out_freq);
 }
 
 // ---------------------------------------------------------------------------

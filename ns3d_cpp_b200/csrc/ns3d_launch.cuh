@@ -22,6 +22,7 @@ struct LaunchCfg {
     int zb;       // planes per block of the 2.5-D viscous kernels (0: from the grid)
     int tiled;    // bit 0: 2.5-D visc_flux (when the box tiles); bit 1: its pipelined form
     long long small;  // FP64 boxes of at most so many cells take k_flux_small (see small_box)
+    int pdl;      // 1: programmatic dependent launches (launch_pdl)
     int pipe;     // FP32 sweeps with the software-pipelined split: bit 0 the x sweep
                   // (k_sweep_x_pipe, rows of >= 128 cells), bit 1 the y / z sweeps (k_sweep_pipe)
 };
@@ -35,15 +36,36 @@ template <class R>
 cudaError_t launch_sweep(const LaunchCfg& L, int dir, StateView W, R* tacc, const Ctrl* ctrl);
 template <class R>
 cudaError_t launch_visc_flux(const LaunchCfg& L, StateView W, R* fv, const Ctrl* ctrl);
-// t3: T_acc as the three separate terms of launch_flux_small.
 template <class R>
 cudaError_t launch_update(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
-                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl, bool t3);
+                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl);
 template <class R>
-cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs, bool t3);
+cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs);
 // All fluxes of an FP64 right-hand side in one launch (k_flux_small): tacc (15
 // blocks of n) and fv. For boxes of small_box() only.
 cudaError_t launch_flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl);
+constexpr long long kSmallUpdateCells = 33000;  // stages of larger boxes: k_update (see k_update_small)
+// The rest of the stage (1 to 3; rhs unused) or of the right-hand side (stage 0;
+// Wc, W0, Wn and ctrl unused) from launch_flux_small's terms.
+cudaError_t launch_update_small(const LaunchCfg& L, int stage, StateView Wc, StateView W0, const double* tacc,
+                                const double* fv, StateOut Wn, Ctrl* ctrl, double* rhs);
+
+// A launch whose kernel calls pdl_wait: with L.pdl it may start while its
+// predecessor in the stream drains.
+template <class... K, class... A>
+cudaError_t launch_pdl(const LaunchCfg& L, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = L.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = L.pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
 // The z sweep fused with the stage update (k_sweep_ring<2, ..., FUSE>): T_acc
 // holds the x + y terms, fv the viscous fluxes of Wc; writes Wn. Component-wise
 // reconstruction only (L.chr == 0; cudaErrorNotSupported otherwise).
@@ -71,11 +93,23 @@ inline int segment_for(int len, long long lines) {
 
 // Whether an FP64 box takes launch_flux_small: component-wise schemes, few
 // enough cells, every line short enough for a block's shared memory, no tuning
-// override of the marching kernels.
+// override of the marching kernels. L.small cells (300000: a step at 64^3
+// 390 -> 335 us, at 96^3 Lax-Friedrichs + MDCD 700 -> 806) for boxes that the
+// warp-per-row x sweep and the tiled viscous flux serve, three times as many for
+// the others (75^3 950 -> 600 us; 130 x 100 x 110, MDCD, 1383 -> 1367).
 inline bool small_box(const LaunchCfg& L) {
     const DevParams& P = L.P;
-    return L.small && !L.chr && P.n <= L.small && P.nx <= SMALL_NC && P.ny <= SMALL_NC && P.nz <= SMALL_NC;
+    const bool tiles = P.nx % 32 == 0 && P.ny % 8 == 0;
+    return L.small && !L.chr && P.n <= (tiles ? L.small : 3 * L.small) && P.nx <= SMALL_NC && P.ny <= SMALL_NC &&
+           P.nz <= SMALL_NC;
 }
+
+// Boxes whose launches overlap by programmatic dependent launch: those whose
+// kernels last some tens of microseconds (FP64 32^3 91 -> 76 us a step, 64^3
+// 391 -> 356 us, FP32 8^3 101 -> 76 us, 96^3 617 -> 585 us). On larger ones the
+// next kernel's waiting blocks cost more than the overlap gains (FP64 128^3 MDCD
+// 1308 -> 1449 us; FP32 112^3 1034 -> 1037).
+inline bool pdl_box(const DevParams& P, bool fp64) { return P.n <= (fp64 ? 300000 : 1000000); }
 
 #ifdef NS3D_LAUNCH_IMPL
 
@@ -111,18 +145,15 @@ cudaError_t sweep_dir(const LaunchCfg& L, StateView W, R* tacc, const Ctrl* ctrl
             if ((L.pipe & 1) && P.nx >= 128) {
                 if constexpr (FVS == FV_SW) {
                     if (P.sw_eps > 0.0) {  // the entropy fix, compiled in
-                        k_sweep_x_pipe<FVS, RC, 1><<<blocks, 32 * XW_WARPS, 0, L.stream>>>(P, W, tacc, ctrl);
-                        return cudaGetLastError();
+                        return launch_pdl(L, k_sweep_x_pipe<FVS, RC, 1>, blocks, 32 * XW_WARPS, 0, P, W, tacc, ctrl);
                     }
                 }
-                k_sweep_x_pipe<FVS, RC, 0><<<blocks, 32 * XW_WARPS, 0, L.stream>>>(P, W, tacc, ctrl);
-                return cudaGetLastError();
+                return launch_pdl(L, k_sweep_x_pipe<FVS, RC, 0>, blocks, 32 * XW_WARPS, 0, P, W, tacc, ctrl);
             }
-            k_sweep_x_warp_f32<FVS, RC><<<blocks, 32 * XW_WARPS, 0, L.stream>>>(P, W, tacc, ctrl);
+            return launch_pdl(L, k_sweep_x_warp_f32<FVS, RC>, blocks, 32 * XW_WARPS, 0, P, W, tacc, ctrl);
+        } else {
+            return launch_pdl(L, k_sweep_x_warp<R, FVS, RC, CHR>, blocks, 32 * XW_WARPS, 0, P, W, tacc, ctrl);
         }
-        else
-            k_sweep_x_warp<R, FVS, RC, CHR><<<blocks, 32 * XW_WARPS, 0, L.stream>>>(P, W, tacc, ctrl);
-        return cudaGetLastError();
     }
     if constexpr (DIR != 0 && !CHR) {
         const MarchShape m = march_shape<DIR>(L, RingCfg<R>::T);
@@ -130,21 +161,17 @@ cudaError_t sweep_dir(const LaunchCfg& L, StateView W, R* tacc, const Ctrl* ctrl
             if (L.pipe & 2) {
                 if constexpr (FVS == FV_SW) {
                     if (P.sw_eps > 0.0) {  // the entropy fix, compiled in
-                        k_sweep_pipe<DIR, FVS, RC, 1><<<m.grid, m.th, 0, L.stream>>>(P, W, tacc, m.seg, ctrl);
-                        return cudaGetLastError();
+                        return launch_pdl(L, k_sweep_pipe<DIR, FVS, RC, 1>, m.grid, m.th, 0, P, W, tacc, m.seg, ctrl);
                     }
                 }
-                k_sweep_pipe<DIR, FVS, RC, 0><<<m.grid, m.th, 0, L.stream>>>(P, W, tacc, m.seg, ctrl);
-                return cudaGetLastError();
+                return launch_pdl(L, k_sweep_pipe<DIR, FVS, RC, 0>, m.grid, m.th, 0, P, W, tacc, m.seg, ctrl);
             }
         }
-        k_sweep_ring<DIR, R, FVS, RC, false><<<m.grid, m.th, 0, L.stream>>>(
+        return launch_pdl(L, k_sweep_ring<DIR, R, FVS, RC, false>, m.grid, m.th, 0,
             P, W, tacc, m.seg, ctrl, FuseArgs<R>{});
-        return cudaGetLastError();
     } else {
         const MarchShape m = march_shape<DIR>(L, 128);
-        k_sweep<DIR, R, FVS, RC, CHR><<<m.grid, m.th, 0, L.stream>>>(P, W, tacc, m.seg, ctrl);
-        return cudaGetLastError();
+        return launch_pdl(L, k_sweep<DIR, R, FVS, RC, CHR>, m.grid, m.th, 0, P, W, tacc, m.seg, ctrl);
     }
 }
 
@@ -152,9 +179,8 @@ template <class R, int FVS, int RC>
 cudaError_t sweep_z_update(const LaunchCfg& L, const FuseArgs<R>& F, StateView Wc,
                            const R* tacc) {
     const MarchShape m = march_shape<2>(L, RingCfg<R>::T);
-    k_sweep_ring<2, R, FVS, RC, true><<<m.grid, m.th, 0, L.stream>>>(
+    return launch_pdl(L, k_sweep_ring<2, R, FVS, RC, true>, m.grid, m.th, 0,
         L.P, Wc, const_cast<R*>(tacc), m.seg, F.ctrl, F);
-    return cudaGetLastError();
 }
 
 // L.chr selects the characteristic-wise sweeps (du_inviscous_character).
@@ -246,8 +272,7 @@ cudaError_t visc_pipe(const LaunchCfg& L, StateView W, R* fv, const Ctrl* ctrl) 
         if (dev >= 0 && dev < 64) opted[dev] = true;
     }
     const dim3 g = grid_25d<R>(L), b(VTile<R>::X, VTile<R>::Y);
-    k_visc_flux_pipe<R, ORD><<<g, b, sm, L.stream>>>(L.P, W, fv, ctrl, zb_for<R>(L));
-    return cudaGetLastError();
+    return launch_pdl(L, k_visc_flux_pipe<R, ORD>, g, b, sm, L.P, W, fv, ctrl, zb_for<R>(L));
 }
 }  // namespace detail
 
@@ -263,68 +288,50 @@ cudaError_t launch_visc_flux(const LaunchCfg& L, StateView W, R* fv, const Ctrl*
     if (detail::tiles_25d<R>(L, 1)) {
         const dim3 g = detail::grid_25d<R>(L), b(VTile<R>::X, VTile<R>::Y);
         switch (L.P.vis_order) {
-        case 4: k_visc_flux_25d<R, 4><<<g, b, 0, L.stream>>>(L.P, W, fv, ctrl, detail::zb_for<R>(L)); break;
-        case 6: k_visc_flux_25d<R, 6><<<g, b, 0, L.stream>>>(L.P, W, fv, ctrl, detail::zb_for<R>(L)); break;
-        default: k_visc_flux_25d<R, 8><<<g, b, 0, L.stream>>>(L.P, W, fv, ctrl, detail::zb_for<R>(L)); break;
+        case 4: return launch_pdl(L, k_visc_flux_25d<R, 4>, g, b, 0, L.P, W, fv, ctrl, detail::zb_for<R>(L));
+        case 6: return launch_pdl(L, k_visc_flux_25d<R, 6>, g, b, 0, L.P, W, fv, ctrl, detail::zb_for<R>(L));
+        default: return launch_pdl(L, k_visc_flux_25d<R, 8>, g, b, 0, L.P, W, fv, ctrl, detail::zb_for<R>(L));
         }
-        return cudaGetLastError();
     }
     const int th = detail::threads_for(L.P.nx);
     const dim3 g = detail::cell_grid(L.P, th);
     switch (L.P.vis_order) {
-    case 4: k_visc_flux<R, 4><<<g, th, 0, L.stream>>>(L.P, W, fv, ctrl); break;
-    case 6: k_visc_flux<R, 6><<<g, th, 0, L.stream>>>(L.P, W, fv, ctrl); break;
-    default: k_visc_flux<R, 8><<<g, th, 0, L.stream>>>(L.P, W, fv, ctrl); break;
+    case 4: return launch_pdl(L, k_visc_flux<R, 4>, g, th, 0, L.P, W, fv, ctrl);
+    case 6: return launch_pdl(L, k_visc_flux<R, 6>, g, th, 0, L.P, W, fv, ctrl);
+    default: return launch_pdl(L, k_visc_flux<R, 8>, g, th, 0, L.P, W, fv, ctrl);
     }
-    return cudaGetLastError();
 }
 
-template <class R, int ORD, bool T3>
+template <class R, int ORD>
 static cudaError_t update_ord(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
                               const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl) {
     const int th = detail::threads_for(L.P.nx);
     const dim3 g = detail::cell_grid(L.P, th);
-    if (stage == 1) k_update<R, ORD, 1, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
-    else if (stage == 2) k_update<R, ORD, 2, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
-    else k_update<R, ORD, 3, T3><<<g, th, 0, L.stream>>>(L.P, Wc, W0, tacc, fv, Wn, ctrl);
-    return cudaGetLastError();
-}
-
-// f(std::bool_constant<T3>): the separate terms exist in the FP64 form only.
-template <class R, class F>
-cudaError_t by_terms(bool t3, F f) {
-    if constexpr (sizeof(R) == 8) {
-        if (t3) return f(std::true_type{});
-    }
-    return f(std::false_type{});
+    if (stage == 1) return launch_pdl(L, k_update<R, ORD, 1>, g, th, 0, L.P, Wc, W0, tacc, fv, Wn, ctrl);
+    if (stage == 2) return launch_pdl(L, k_update<R, ORD, 2>, g, th, 0, L.P, Wc, W0, tacc, fv, Wn, ctrl);
+    return launch_pdl(L, k_update<R, ORD, 3>, g, th, 0, L.P, Wc, W0, tacc, fv, Wn, ctrl);
 }
 
 template <class R>
 cudaError_t launch_update(const LaunchCfg& L, int stage, StateView Wc, StateView W0,
-                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl, bool t3) {
-    return by_terms<R>(t3, [&](auto t) -> cudaError_t {
-        constexpr bool T3 = decltype(t)::value;
-        switch (L.P.vis_order) {
-        case 4: return update_ord<R, 4, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-        case 6: return update_ord<R, 6, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-        default: return update_ord<R, 8, T3>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
-        }
-    });
+                          const R* tacc, const R* fv, StateOut Wn, Ctrl* ctrl) {
+    switch (L.P.vis_order) {
+    case 4: return update_ord<R, 4>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+    case 6: return update_ord<R, 6>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+    default: return update_ord<R, 8>(L, stage, Wc, W0, tacc, fv, Wn, ctrl);
+    }
 }
 
 template <class R>
-cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs, bool t3) {
+cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, double* rhs) {
     const int th = detail::threads_for(L.P.nx);
     const dim3 g = detail::cell_grid(L.P, th);
-    return by_terms<R>(t3, [&](auto t) -> cudaError_t {
-        constexpr bool T3 = decltype(t)::value;
-        switch (L.P.vis_order) {
-        case 4: k_rhs_out<R, 4, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
-        case 6: k_rhs_out<R, 6, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
-        default: k_rhs_out<R, 8, T3><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
-        }
-        return cudaGetLastError();
-    });
+    switch (L.P.vis_order) {
+    case 4: k_rhs_out<R, 4><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+    case 6: k_rhs_out<R, 6><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+    default: k_rhs_out<R, 8><<<g, th, 0, L.stream>>>(L.P, tacc, fv, rhs); break;
+    }
+    return cudaGetLastError();
 }
 
 #ifdef NS3D_LAUNCH_SMALL
@@ -360,8 +367,7 @@ cudaError_t flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv
         nc = c > nc ? c : nc;
     }
     const unsigned blocks = (unsigned)(sh.nb[0] + sh.nb[1] + sh.nb[2] + sh.nb[3]);
-    k_flux_small<FVS, RC><<<blocks, SMALL_T, small_smem(nc), L.stream>>>(L.P, W, tacc, fv, sh, ctrl);
-    return cudaGetLastError();
+    return launch_pdl(L, k_flux_small<FVS, RC>, blocks, SMALL_T, small_smem(nc), L.P, W, tacc, fv, sh, ctrl);
 }
 }  // namespace detail
 
@@ -380,14 +386,48 @@ cudaError_t launch_flux_small(const LaunchCfg& L, StateView W, double* tacc, dou
     return L.fvs == FV_SW ? by_rc(std::integral_constant<int, FV_SW>{})
                           : by_rc(std::integral_constant<int, FV_LF>{});
 }
+
+template <int ORD>
+static cudaError_t update_small_ord(const LaunchCfg& L, int stage, StateView Wc, StateView W0, const double* tacc,
+                                    const double* fv, StateOut Wn, Ctrl* ctrl, double* rhs) {
+    const unsigned blocks = (unsigned)((L.P.n + 31) / 32);
+    if (stage > 0 && L.P.n > kSmallUpdateCells) {
+        const int th = detail::threads_for(L.P.nx);
+        const dim3 g = detail::cell_grid(L.P, th);
+        auto wide = [&](auto st) {
+            return launch_pdl(L, k_update<double, ORD, decltype(st)::value, true>, g, th, 0, L.P, Wc, W0, tacc, fv, Wn,
+                              ctrl);
+        };
+        if (stage == 1) return wide(std::integral_constant<int, 1>{});
+        if (stage == 2) return wide(std::integral_constant<int, 2>{});
+        return wide(std::integral_constant<int, 3>{});
+    }
+    auto go = [&](auto st) {
+        return launch_pdl(L, k_update_small<ORD, decltype(st)::value>, blocks, 160, 0, L.P, Wc, W0, tacc, fv, Wn,
+                          ctrl, rhs);
+    };
+    if (stage == 0) return go(std::integral_constant<int, 0>{});
+    if (stage == 1) return go(std::integral_constant<int, 1>{});
+    if (stage == 2) return go(std::integral_constant<int, 2>{});
+    return go(std::integral_constant<int, 3>{});
+}
+
+cudaError_t launch_update_small(const LaunchCfg& L, int stage, StateView Wc, StateView W0, const double* tacc,
+                                const double* fv, StateOut Wn, Ctrl* ctrl, double* rhs) {
+    switch (L.P.vis_order) {
+    case 4: return update_small_ord<4>(L, stage, Wc, W0, tacc, fv, Wn, ctrl, rhs);
+    case 6: return update_small_ord<6>(L, stage, Wc, W0, tacc, fv, Wn, ctrl, rhs);
+    default: return update_small_ord<8>(L, stage, Wc, W0, tacc, fv, Wn, ctrl, rhs);
+    }
+}
 #endif  // NS3D_LAUNCH_SMALL
 
 #define NS3D_INSTANTIATE_LAUNCHERS(R)                                                          \
     template cudaError_t launch_sweep<R>(const LaunchCfg&, int, StateView, R*, const Ctrl*);   \
     template cudaError_t launch_visc_flux<R>(const LaunchCfg&, StateView, R*, const Ctrl*);    \
     template cudaError_t launch_update<R>(const LaunchCfg&, int, StateView, StateView,         \
-                                          const R*, const R*, StateOut, Ctrl*, bool);          \
-    template cudaError_t launch_rhs_out<R>(const LaunchCfg&, const R*, const R*, double*, bool); \
+                                          const R*, const R*, StateOut, Ctrl*);                \
+    template cudaError_t launch_rhs_out<R>(const LaunchCfg&, const R*, const R*, double*);   \
     template cudaError_t launch_sweep_z_update<R>(const LaunchCfg&, int, StateView, StateView, \
                                                   const R*, const R*, StateOut, Ctrl*);
 

@@ -31,10 +31,10 @@ using namespace ns3d;
 namespace ns3d {
 extern template cudaError_t launch_sweep<double>(const LaunchCfg&, int, StateView, double*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<double>(const LaunchCfg&, StateView, double*, const Ctrl*);
-extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*, bool);
+extern template cudaError_t launch_rhs_out<double>(const LaunchCfg&, const double*, const double*, double*);
 extern template cudaError_t launch_sweep<float>(const LaunchCfg&, int, StateView, float*, const Ctrl*);
 extern template cudaError_t launch_visc_flux<float>(const LaunchCfg&, StateView, float*, const Ctrl*);
-extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*, bool);
+extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*);
 }  // namespace ns3d
 
 // 15 doubles per cell: T (double) + 5 accumulator values + the viscous fluxes
@@ -96,13 +96,18 @@ cudaError_t rhs_into(const LaunchCfg& L, StateView W, double* scratch, double* r
     R* fv = reinterpret_cast<R*>((reinterpret_cast<uintptr_t>(tacc + (t3 ? 15 : 5) * n) + 15) & ~uintptr_t(15));
     cudaError_t e = cudaSuccess;
     if constexpr (sizeof(R) == 8) {
-        if (t3) e = launch_flux_small(L, W, tacc, fv, nullptr);
+        if (t3) {
+            e = launch_flux_small(L, W, tacc, fv, nullptr);
+            if (e == cudaSuccess)
+                e = launch_update_small(L, 0, StateView{}, StateView{}, tacc, fv, StateOut{}, nullptr, rhs);
+            return e;
+        }
     }
-    if (!t3) {
+    {
         for (int dir = 0; dir < 3 && e == cudaSuccess; ++dir) e = launch_sweep<R>(L, dir, W, tacc, nullptr);
         if (e == cudaSuccess) e = launch_visc_flux<R>(L, W, fv, nullptr);
     }
-    if (e == cudaSuccess) e = launch_rhs_out<R>(L, tacc, fv, rhs, t3);
+    if (e == cudaSuccess) e = launch_rhs_out<R>(L, tacc, fv, rhs);
     return e;
 }
 

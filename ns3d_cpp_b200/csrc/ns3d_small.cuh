@@ -117,6 +117,7 @@ template <int FVS, int RC>
 __global__ void __launch_bounds__(SMALL_T, 512 / SMALL_T)
 k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restrict__ fv, SmallShape sh,
              const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
     if (ctrl && ctrl->stop) return;
     extern __shared__ double small_sm[];
     const long long n = P.n;
@@ -142,6 +143,67 @@ k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restri
     if (P.vis_order == 4) visc_cell<double, 4>(P, W, fv, i, j, k);
     else if (P.vis_order == 6) visc_cell<double, 6>(P, W, fv, i, j, k);
     else visc_cell<double, 8>(P, W, fv, i, j, k);
+}
+
+// The rest of a stage (STAGE 1 to 3, k_update's operations) or of a right-hand
+// side (STAGE 0, k_rhs_out's) of a small box: 32 cells by five warps. Warps 0 to
+// 3 take the viscous divergence of one momentum or energy component each and
+// the fifth the two conserved states, then the stage: a quarter of k_update's 96
+// neighbour loads per thread one after the other, which is what bounds it there
+// (a stage at 16^3: 6 us against 8; from 48^3 on k_update's larger number of
+// cells in flight is the better one; four warps, with the stage in warp 0,
+// measured 2% slower than five).
+template <int ORD, int STAGE>
+__global__ void __launch_bounds__(160)
+k_update_small(DevParams P, StateView Wc, StateView W0, const double* __restrict__ t3,
+               const double* __restrict__ fv, StateOut Wn, Ctrl* ctrl, double* __restrict__ rhs) {
+    pdl_wait();
+    if constexpr (STAGE > 0) {
+        pdl_trigger();
+        if (ctrl->stop) return;
+    }
+    __shared__ double rs[5][32];
+    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+    const long long n = P.n;
+    const int cell = blockIdx.x * 32 + lane;
+    const bool live = cell < n;
+    const long long id = live ? cell : 0;
+    double r = 0.0;
+    if (wq < 4) {
+        const int nx = P.nx, ny = P.ny, nz = P.nz;
+        const int i = (int)(id % nx), jk = (int)(id / nx), j = jk % ny, k = jk / ny;
+        const long long sxy = (long long)nx * ny;
+        // flux blocks of component wq + 1 along x, y, z (see cell_visc)
+        const double* X = fv + (wq == 0 ? 0 : (wq == 1 ? 3 : (wq == 2 ? 4 : 6))) * n + id;
+        const double* Y = fv + (wq == 0 ? 3 : (wq == 1 ? 1 : (wq == 2 ? 5 : 7))) * n + id;
+        const double* Z = fv + (wq == 0 ? 4 : (wq == 1 ? 5 : (wq == 2 ? 2 : 8))) * n + id;
+        r += dcentral_dir<double, ORD>(P, 0, [&](int o) { return X[wrap1(i + o, nx) - i]; }, P.dx);
+        r += dcentral_dir<double, ORD>(P, 1, [&](int o) { return Y[(long long)(wrap1(j + o, ny) - j) * nx]; }, P.dy);
+        r += dcentral_dir<double, ORD>(P, 2, [&](int o) { return Z[(long long)(wrap1(k + o, nz) - k) * sxy]; }, P.dz);
+    }
+    const int q = wq < 4 ? wq + 1 : 0;
+    r += -acc_term<double, true>(t3, n, q, id);
+    if constexpr (STAGE == 0) {
+        if (live) rhs[q * n + id] = r;
+    } else {
+        double U0[5], U[5];
+        if (wq == 4) stage_load<double, STAGE>(P, Wc, W0, id, U0, U);
+        else rs[q][lane] = r;
+        __syncthreads();
+        if (wq < 4) return;
+        const double rc[5] = {r, rs[1][lane], rs[2][lane], rs[3][lane], rs[4][lane]};
+        double cand = CFL_INIT;
+        if (live) stage_apply<double, STAGE>(P, U0, U, id, rc, ctrl->dt, Wn, ctrl, cand);
+        if constexpr (STAGE == 3) {
+            unsigned long long b = (cand == cand) ? pos_double_bits(cand) : ~0ull;  // NaN never wins
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long x = __shfl_xor_sync(0xffffffffu, b, o);
+                b = x < b ? x : b;
+            }
+            if (lane == 0 && b != ~0ull) atomicMin(&ctrl->dtmin_bits, b);
+        }
+    }
 }
 
 }  // namespace ns3d

@@ -103,6 +103,35 @@ def test_noalloc_either_side_of_the_separate_terms(n):
     assert np.array_equal(rhs.cpu().numpy(), want)
 
 
+def test_noalloc_captured_in_a_graph():
+    """The entry point enqueues on the caller's stream only, so it can be
+    captured (after a first call); a replay on new inputs gives their result."""
+    import ctypes
+    import torch
+    from ns3d_cpp_b200 import _lib
+    box = (20, 18, 16)
+    p = _box_params(box)
+    d = torch.from_numpy(_field(box)).cuda()
+    rhs = torch.empty_like(d)
+
+    def call(out):
+        st = _lib.load().ns3d_compute_rhs_noalloc(ctypes.byref(p), *[d[q].data_ptr() for q in range(5)],
+                                                  out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+
+    call(rhs)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        call(rhs)
+    d.copy_(torch.from_numpy(_field(box, seed=9)))
+    g.replay()
+    want = torch.empty_like(d)
+    torch.cuda.synchronize()
+    call(want)
+    torch.cuda.synchronize()
+    assert torch.equal(rhs, want) and bool(torch.isfinite(rhs).all())
+
+
 EXTREME = [("p", 1e160), ("p", np.inf), ("u", np.nan), ("u", 1e200), ("rho", 1e305),
            ("w", -np.inf), ("p", -1.0), ("p", 0.0)]
 
