@@ -755,7 +755,7 @@ void default_tiling(LaunchCfg& L) {
     L.tiled = 3;  // 2.5-D viscous flux, pipelined plane loads (k_visc_flux_pipe)
     L.pipe = 3;   // FP32 sweeps with the software-pipelined split (k_sweep_x_pipe, k_sweep_pipe)
     // an override of the marching kernels' shapes selects those kernels
-    L.small = 300000;
+    L.small = 1500000;
     L.pdl = 1;  // where pdl_box() holds
     if (const char* e = std::getenv("NS3D_PDL")) L.pdl = std::atoi(e);
     for (const char* v : {"NS3D_TILE_ZB", "NS3D_TILED", "NS3D_SEG"})
@@ -845,7 +845,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     ctx->L.chr = q.char_recon ? 1 : 0;
     for (int d = 0; d < 3; ++d) ctx->L.seg[d] = 0;  // chosen per launch from the grid
     default_tiling(ctx->L);
-    if (!pdl_box(P, q.precision == NS3D_PREC_FP64)) ctx->L.pdl = 0;
+    if (!pdl_box(ctx->L, q.precision == NS3D_PREC_FP64)) ctx->L.pdl = 0;
     ctx->rsize = q.precision == NS3D_PREC_FP64 ? sizeof(double) : sizeof(float);
 
     auto bail = [&](ns3d_status st, const std::string& m) {

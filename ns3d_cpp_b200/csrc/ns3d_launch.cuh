@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "ns3d_kernels.cuh"
@@ -91,25 +92,33 @@ inline int segment_for(int len, long long lines) {
 
 }  // namespace detail
 
-// Whether an FP64 box takes launch_flux_small: component-wise schemes, few
-// enough cells, every line short enough for a block's shared memory, no tuning
-// override of the marching kernels. L.small cells (300000: a step at 64^3
-// 390 -> 335 us, at 96^3 Lax-Friedrichs + MDCD 700 -> 806) for boxes that the
-// warp-per-row x sweep and the tiled viscous flux serve, three times as many for
-// the others (75^3 950 -> 600 us; 130 x 100 x 110, MDCD, 1383 -> 1367).
+// Whether an FP64 box takes launch_flux_small: component-wise schemes, every
+// line short enough for a block's shared memory, no tuning override of the
+// marching kernels, and few enough cells: L.small (1500000) where nx is a
+// multiple of 32 and the x sweep marches a warp per row (a step at 64^3 356 ->
+// 265 us, 112^3 1917 -> 1508 us WENO5 and 1214 -> 1044 us MDCD; 128^3 2092 -> 2102
+// and 1319 -> 1456), six times as many elsewhere, where it marches a thread per
+// row (100x75x90 1203 -> 773 us, 200^3 10.2 -> 8.6 ms WENO5, 6.6 -> 6.2 ms MDCD;
+// larger ones not measured).
 inline bool small_box(const LaunchCfg& L) {
     const DevParams& P = L.P;
-    const bool tiles = P.nx % 32 == 0 && P.ny % 8 == 0;
-    return L.small && !L.chr && P.n <= (tiles ? L.small : 3 * L.small) && P.nx <= SMALL_NC && P.ny <= SMALL_NC &&
-           P.nz <= SMALL_NC;
+    return L.small && !L.chr && P.n <= (P.nx % 32 == 0 ? L.small : 6 * L.small) && P.nx <= SMALL_NC &&
+           P.ny <= SMALL_NC && P.nz <= SMALL_NC;
 }
 
 // Boxes whose launches overlap by programmatic dependent launch: those whose
 // kernels last some tens of microseconds (FP64 32^3 91 -> 76 us a step, 64^3
-// 391 -> 356 us, FP32 8^3 101 -> 76 us, 96^3 617 -> 585 us). On larger ones the
-// next kernel's waiting blocks cost more than the overlap gains (FP64 128^3 MDCD
-// 1308 -> 1449 us; FP32 112^3 1034 -> 1037).
-inline bool pdl_box(const DevParams& P, bool fp64) { return P.n <= (fp64 ? 300000 : 1000000); }
+// 281 -> 266 us; FP32 8^3 101 -> 76 us, 64^3 243 -> 212 us, 96^3 616 -> 587 us). On
+// larger ones the next kernel's waiting blocks cost more than the overlap gains
+// (FP64 128^3 MDCD 1308 -> 1449 us, FP32 90x100x84 651 -> 665), in the FP32
+// form's eight-point schemes earlier (75^3 455 -> 520 us, 64^3 228 -> 197).
+inline bool pdl_box(const LaunchCfg& L, bool fp64) {
+    const long long n = L.P.n;
+    if (n <= 30000) return true;
+    if (L.chr || L.rc == RC_MDCD_HYBRID) return false;
+    if (fp64) return n <= 300000;
+    return n <= 700000 && (L.rc != RC_LIN8 || (L.P.nx % 32 == 0 && n <= 300000));
+}
 
 #ifdef NS3D_LAUNCH_IMPL
 
@@ -336,37 +345,13 @@ cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, doubl
 
 #ifdef NS3D_LAUNCH_SMALL
 namespace detail {
-inline SmallShape small_shape(const LaunchCfg& L) {
-    const DevParams& P = L.P;
-    SmallShape sh{};
-    // lines per block: 64 to 256 cells, so that the three sweeps give at least
-    // two blocks per SM; four lines or more along y and z (32-byte rows)
-    long long target = 3 * P.n / (2 * 148);
-    target = target < 64 ? 64 : (target > 256 ? 256 : target);
-    for (int d = 0; d < 3; ++d) {
-        const int len = d == 0 ? P.nx : (d == 1 ? P.ny : P.nz);
-        const long long lines = d == 0 ? (long long)P.ny * P.nz : P.nx;
-        long long lb = (target + len / 2) / len;
-        if (d > 0 && lb < 4) lb = 4;
-        if (lb > SMALL_NC / len) lb = SMALL_NC / len;
-        if (lb > lines) lb = lines;
-        if (lb < 1) lb = 1;
-        sh.lb[d] = (int)lb;
-        sh.nb[d] = (int)((lines + lb - 1) / lb) * (d == 0 ? 1 : (d == 1 ? P.nz : P.ny));
-    }
-    sh.nb[3] = (int)((P.n + SMALL_T - 1) / SMALL_T);
-    return sh;
-}
-
 template <int FVS, int RC>
 cudaError_t flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
-    const SmallShape sh = small_shape(L);
-    int nc = 0;
-    for (int d = 0; d < 3; ++d) {
-        const int c = sh.lb[d] * (d == 0 ? L.P.nx : (d == 1 ? L.P.ny : L.P.nz));
-        nc = c > nc ? c : nc;
-    }
-    const unsigned blocks = (unsigned)(sh.nb[0] + sh.nb[1] + sh.nb[2] + sh.nb[3]);
+    // 64 to 256 cells a block, so that the three sweeps give at least two blocks per SM
+    const long long target = std::min(256ll, std::max(64ll, 3 * L.P.n / (2 * 148)));
+    const SmallShape sh = small_shape(L.P, target, SMALL_NC, SMALL_T);
+    const int nc = small_cells(L.P, sh);
+    const unsigned blocks = small_blocks(sh);
     return launch_pdl(L, k_flux_small<FVS, RC>, blocks, SMALL_T, small_smem(nc), L.P, W, tacc, fv, sh, ctrl);
 }
 }  // namespace detail

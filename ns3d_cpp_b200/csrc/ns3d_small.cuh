@@ -5,11 +5,13 @@
 // one thread splits S cells and reconstructs its faces one after the other, the
 // launches depend on each other through T_acc, and a 32^3 box has 1024 lines
 // for 148 SMs. Here a block takes a few whole periodic lines into shared
-// memory: every thread splits one cell, then reconstructs one component of one
-// face (five times the parallelism, no halo cells, no serial march), then
-// differences. Each direction writes its own term, so nothing depends on
-// another launch; the reader adds them in T_acc's order (acc_term). The
-// operations per cell and face are those of the marching kernels: same bits.
+// memory: every thread splits one cell, then reconstructs the face on its right
+// (no halo cells, no serial march), then differences. Each direction writes its
+// own term, so nothing depends on another launch; the reader adds them in
+// T_acc's order (acc_term). The operations per cell and face are those of the
+// marching kernels: same bits. A thread takes the components of a face in a
+// loop, so that the slot arithmetic is paid once for five (a step at 64^3 315 ->
+// 266 us; the FP64 pipe was 54% busy, issue 62%).
 //
 // FP64 only: the FP32 form's reconstructions work on float deviations from an
 // offset per marching segment, and its roundings belong to the marching kernels.
@@ -30,6 +32,75 @@ struct SmallShape {
     int nb[4], lb[3];
 };
 
+// `target` cells per block (lines of up to `most` cells), four lines or more
+// along y and z (32-byte rows); `vth` cells per block of the fourth role.
+inline SmallShape small_shape(const DevParams& P, long long target, int most, int vth) {
+    SmallShape sh{};
+    for (int d = 0; d < 3; ++d) {
+        const int len = d == 0 ? P.nx : (d == 1 ? P.ny : P.nz);
+        const long long lines = d == 0 ? (long long)P.ny * P.nz : P.nx;
+        long long lb = (target + len / 2) / len;
+        if (d > 0 && lb < 4) lb = 4;
+        if (lb > most / len) lb = most / len;
+        if (lb > lines) lb = lines;
+        if (lb < 1) lb = 1;
+        sh.lb[d] = (int)lb;
+        sh.nb[d] = (int)((lines + lb - 1) / lb) * (d == 0 ? 1 : (d == 1 ? P.nz : P.ny));
+    }
+    sh.nb[3] = (int)((P.n + vth - 1) / vth);
+    return sh;
+}
+// Cells of the largest block of the shape, blocks of the launch.
+inline int small_cells(const DevParams& P, const SmallShape& sh) {
+    const int c[3] = {sh.lb[0] * P.nx, sh.lb[1] * P.ny, sh.lb[2] * P.nz};
+    const int m = c[0] > c[1] ? c[0] : c[1];
+    return m > c[2] ? m : c[2];
+}
+inline unsigned small_blocks(const SmallShape& sh) {
+    return (unsigned)sh.nb[0] + (unsigned)sh.nb[1] + (unsigned)sh.nb[2] + (unsigned)sh.nb[3];
+}
+
+// The whole lines along DIR of block b of a role with lb lines per block: line
+// l, position s is cell id0 + l dl + s ds and slot l cl + s cs of the block's
+// nc = nl len slots (slots consecutive in memory order: coalesced).
+template <int DIR>
+struct LineTile {
+    long long id0, dl, ds;
+    int nl, len, cl, cs, nc;
+    unsigned rd;  // ceil(2^32 / d), d the divisor of of_slot: c / d = umulhi(c, rd) for c, d < 2^16
+    __device__ __forceinline__ LineTile(const DevParams& P, int b, int lb) {
+        const int nx = P.nx, ny = P.ny, nz = P.nz;
+        len = DIR == 0 ? nx : (DIR == 1 ? ny : nz);
+        if constexpr (DIR == 0) {
+            const int l0 = b * lb;
+            nl = min(lb, ny * nz - l0);
+            id0 = (long long)l0 * nx; dl = nx; ds = 1;
+        } else {
+            const int gx = (nx + lb - 1) / lb, o = b / gx, i0 = (b - o * gx) * lb;
+            nl = min(lb, nx - i0);
+            id0 = (DIR == 1 ? (long long)o * ny : (long long)o) * nx + i0;
+            dl = 1;
+            ds = DIR == 1 ? (long long)nx : (long long)nx * ny;
+        }
+        cl = DIR == 0 ? len : 1;
+        cs = DIR == 0 ? 1 : nl;
+        nc = nl * len;
+        rd = 0xffffffffu / (unsigned)(DIR == 0 ? len : nl) + 1u;  // 0 for d = 1
+    }
+    __device__ __forceinline__ void of_slot(int c, int& l, int& s) const {
+        if constexpr (DIR == 0) {
+            l = (int)__umulhi((unsigned)c, rd);  // len >= 8
+            s = c - l * len;
+        } else {
+            s = rd == 0u ? c : (int)__umulhi((unsigned)c, rd);
+            l = c - s * nl;
+        }
+    }
+    __device__ __forceinline__ long long id(int l, int s) const { return id0 + l * dl + s * ds; }
+    // slot offset of position s (periodic, within a line length of the line)
+    __device__ __forceinline__ int at(int s) const { return wrap1(s, len) * cs; }
+};
+
 constexpr int small_smem(int nc) { return nc * 15 * (int)sizeof(double); }
 
 // The sweep along DIR of the lines of block b: out (5 blocks of n).
@@ -38,35 +109,15 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
                                             double* __restrict__ out, int b, int lb, double* sm) {
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long n = P.n;
-    const int len = DIR == 0 ? nx : (DIR == 1 ? ny : nz);
-    // line l of the block, position s: cell id0 + l dl + s ds, slot l cl + s cs
-    long long id0, dl, ds;
-    int nl;
-    if constexpr (DIR == 0) {
-        const int l0 = b * lb;
-        nl = min(lb, ny * nz - l0);
-        id0 = (long long)l0 * nx; dl = nx; ds = 1;
-    } else {
-        const int gx = (nx + lb - 1) / lb, o = b / gx, i0 = (b - o * gx) * lb;
-        nl = min(lb, nx - i0);
-        id0 = (DIR == 1 ? (long long)o * ny : (long long)o) * nx + i0;
-        dl = 1;
-        ds = DIR == 1 ? (long long)nx : (long long)nx * ny;
-    }
-    const int cl = DIR == 0 ? len : 1, cs = DIR == 0 ? 1 : nl;
-    const int nc = nl * len;
+    const LineTile<DIR> tl(P, b, lb);
+    const int nc = tl.nc;
     double* F = sm;             // [10][nc]: F+0..4, F-0..4
     double* fl = sm + 10 * nc;  // [5][nc]: face right of each cell
-    auto line_of_slot = [&](int c, int& l, int& s) {
-        if constexpr (DIR == 0) { l = c / len; s = c - l * len; }
-        else { s = c / nl; l = c - s * nl; }
-    };
     for (int c = threadIdx.x; c < nc; c += SMALL_T) {
         int l, s;
-        line_of_slot(c, l, s);
-        const long long id = id0 + l * dl + s * ds;
+        tl.of_slot(c, l, s);
+        const long long id = tl.id(l, s);
         const double raw[5] = {W.rho[id], W.u[id], W.v[id], W.w[id], W.p[id]};
         double Fp[5], Fm[5];
         split_fp64<FVS, RC, DIR == 0, DIR == 1, DIR == 2>(P, raw, Fp, Fm);
@@ -77,37 +128,48 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
         }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < 5 * nc; t += SMALL_T) {
-        // component q of the face between positions s and s+1 of line l
-        const int q = t / nc, c = t - q * nc;
+    // a thread takes a face's components one after the other; of a block with no
+    // more cells than half its threads two threads share them
+    const bool two = nc <= SMALL_T / 2;
+    const int half = two && threadIdx.x >= SMALL_T / 2 ? 1 : 0;
+    const int q0 = half ? 3 : 0, q1 = two && !half ? 3 : 5;
+    for (int c = threadIdx.x - half * (SMALL_T / 2); c < nc; c += SMALL_T) {
+        // the face between positions s and s+1 of line l
         int l, s;
-        line_of_slot(c, l, s);
-        const double* fp = F + q * nc + l * cl;
-        const double* fm = fp + 5 * nc;
-        double a[S], bm[S];
+        tl.of_slot(c, l, s);
+        int w[S];
 #pragma unroll
-        for (int m = 0; m < S; ++m) {
-            const int w = wrap1(s - MID + m, len) * cs;
-            a[m] = fp[w];
-            bm[S - 1 - m] = fm[w];  // reconstruct_select reverses for flag < 0
+        for (int m = 0; m < S; ++m) w[m] = tl.at(s - MID + m) + l * tl.cl;
+#pragma unroll 1
+        for (int q = q0; q < q1; ++q) {
+            const double* fp = F + q * nc;
+            const double* fm = fp + 5 * nc;
+            double a[S], bm[S];
+#pragma unroll
+            for (int m = 0; m < S; ++m) {
+                a[m] = fp[w[m]];
+                bm[S - 1 - m] = fm[w[m]];  // reconstruct_select reverses for flag < 0
+            }
+            double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
+                       reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
+            if constexpr (RC == RC_WENO5) {  // as in recon_face
+                if (!finite_hi(f))
+                    f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
+                        weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
+            }
+            fl[q * nc + c] = f;
         }
-        double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
-                   reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
-        if constexpr (RC == RC_WENO5) {  // as in recon_face
-            if (!finite_hi(f))
-                f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
-                    weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
-        }
-        fl[t] = f;
+        if (two) break;
     }
     __syncthreads();
     const double inv_h = DIR == 0 ? P.inv_dx : (DIR == 1 ? P.inv_dy : P.inv_dz);
-    for (int t = threadIdx.x; t < 5 * nc; t += SMALL_T) {
-        const int q = t / nc, c = t - q * nc;
+    for (int c = threadIdx.x; c < nc; c += SMALL_T) {
         int l, s;
-        line_of_slot(c, l, s);
-        const double d = fl[t] - fl[q * nc + l * cl + wrap1(s - 1, len) * cs];
-        out[q * n + id0 + l * dl + s * ds] = d * inv_h;
+        tl.of_slot(c, l, s);
+        const int left = l * tl.cl + tl.at(s - 1);
+        double* o = out + tl.id(l, s);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) o[q * n] = (fl[q * nc + c] - fl[q * nc + left]) * inv_h;
     }
 }
 
