@@ -232,7 +232,7 @@ ns3d_status ns3d_step_dts(ns3d_ctx *ctx, int nsteps, const double *dts);
  * kinetic energy sum 0.5 rho |u|^2 dV of compute_total_energy
  * (postprocess.cpp:103), whose value is returned in *J. grad receives dJ/dw
  * at the start state. The forward run stores the state every
- * `checkpoint_every` steps; the reverse sweep recomputes each segment's stage
+ * `checkpoint_every` steps; the reverse sweep recomputes each earlier segment's stage
  * states from its checkpoint. Afterwards the context holds the end state. */
 ns3d_status ns3d_adjoint(ns3d_ctx *ctx, int nsteps, int checkpoint_every, const double *dts,
                          double *dts_out, const double *lam_final, double *grad, double *J);

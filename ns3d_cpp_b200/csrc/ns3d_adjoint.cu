@@ -4,13 +4,16 @@
 //
 // RHS VJP, per direction d (R = V - sum_d inv_h_d (F_d(f) - F_d(f-1))):
 //   lamF(f) = inv_h (lamR(f+1) - lamR(f))                     (face f = f+1/2)
-//   k_adj_face: reconstruction VJP of every face into G (2 x S x 5 arrays)
-//   k_adj_cell: lamF+-(c) = sum over the faces whose windows hold c, then the
-//               transposed split Jacobian -> lamW(c) +=
+//   reconstruction VJP of every face, lamF+-(c) = sum over the faces whose
+//   windows hold c, then the transposed split Jacobian: k_adj_flux in shared
+//   memory; for lines too long for that k_adj_face (the window cotangents into
+//   G, 2 x S x 5 arrays) and k_adj_cell (the gather)
 // Viscous part: lam of the fluxes = D^T lamR = -D lamR (antisymmetric central
 // stencils on a periodic line), pointwise flux VJP (tau, q, mu(T)), then the
 // gradient transpose -D again.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "ns3d_adjoint.cuh"
 #include "ns3d_internal.h"
@@ -142,10 +145,10 @@ k_adj_face(DevParams P, StateView W, const double* __restrict__ lamR, double* __
 }
 
 // Gather of the split-flux cotangents of each cell and the transposed split
-// Jacobian: lamW(c) += (dF+/dw)^T lamF+(c) + (dF-/dw)^T lamF-(c).
+// Jacobian: out(c) = (dF+/dw)^T lamF+(c) + (dF-/dw)^T lamF-(c).
 template <int DIR, int FVS, int RC>
 __global__ void __launch_bounds__(128)
-k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __restrict__ lamW) {
+k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __restrict__ out) {
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
     // x: threads over j (G's x layout is j-fastest); y, z: threads over i
@@ -180,20 +183,17 @@ k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __res
     load_w5(W, id, w5);
     split_vjp<FVS, DIR>(w5, P.gamma, P.sw_eps, gp, gm, gw);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) lamW[q * n + id] += gw[q];
+    for (int q = 0; q < 5; ++q) out[q * n + id] = gw[q];
 }
 
 // Viscous VJP, part 1: lam of the 12 gradients and the direct lam of u,v,w,T.
 // lg blocks: 0..11 gradients (du/dx du/dy du/dz dv/.. dw/.. dT/..), 12..15 u,v,w,T.
 template <int ORD>
-__global__ void __launch_bounds__(128)
-k_adj_visc1(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ lg) {
-    const int nx = P.nx, ny = P.ny, nz = P.nz;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
+__device__ __forceinline__ void adj_visc1_cell(const DevParams& P, const StateView& W,
+                                               const double* __restrict__ lamR,
+                                               double* __restrict__ lg, int i, int j, int k) {
     const long long n = P.n;
-    const long long id = ((long long)k * ny + j) * nx + i;
+    const long long id = ((long long)k * P.ny + j) * P.nx + i;
     const Line Lx = line_of<0>(P, i, j, k, id), Ly = line_of<1>(P, i, j, k, id),
                Lz = line_of<2>(P, i, j, k, id);
     auto d = [&](const double* a, const Line& L, double h) {
@@ -253,15 +253,13 @@ k_adj_visc1(DevParams P, StateView W, const double* __restrict__ lamR, double* _
 }
 
 // Viscous VJP, part 2: gradient transpose (-D) plus the direct parts; T = p/(rho R).
+// Added to the cotangent lw of one cell.
 template <int ORD>
-__global__ void __launch_bounds__(128)
-k_adj_visc2(DevParams P, StateView W, const double* __restrict__ lg, double* __restrict__ lamW) {
-    const int nx = P.nx, ny = P.ny;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    const int j = blockIdx.y, k = blockIdx.z;
+__device__ __forceinline__ void adj_visc2_cell(const DevParams& P, const StateView& W,
+                                               const double* __restrict__ lg, int i, int j, int k,
+                                               double lw[5]) {
     const long long n = P.n;
-    const long long id = ((long long)k * ny + j) * nx + i;
+    const long long id = ((long long)k * P.ny + j) * P.nx + i;
     const Line Lx = line_of<0>(P, i, j, k, id), Ly = line_of<1>(P, i, j, k, id),
                Lz = line_of<2>(P, i, j, k, id);
     auto d = [&](int blk, const Line& L, double h) {
@@ -276,35 +274,193 @@ k_adj_visc2(DevParams P, StateView W, const double* __restrict__ lg, double* __r
     double rr = W.rho[id];
     if (rr <= 0.0) rr = 1e-12;
     const double T = W.T[id];
-    lamW[1 * n + id] += lv4[0];
-    lamW[2 * n + id] += lv4[1];
-    lamW[3 * n + id] += lv4[2];
-    lamW[4 * n + id] += lv4[3] / (rr * P.Rgas);
-    lamW[0 * n + id] += -lv4[3] * T / rr;
+    lw[1] += lv4[0];
+    lw[2] += lv4[1];
+    lw[3] += lv4[2];
+    lw[4] += lv4[3] / (rr * P.Rgas);
+    lw[0] += -lv4[3] * T / rr;
+}
+
+// ---------------------------------------------------------------------------
+// The RHS VJP in two launches.
+//
+// k_adj_flux: blocks of whole lines (LineTile) along x, y and z and, beside
+// them, the first viscous part. A block splits its cells once into shared
+// memory; then, one component at a time, every thread takes the
+// reconstruction VJP of a face and, after a barrier, sums its cell's cotangents
+// from the faces around it; the cell's ten sums end in the split Jacobian. The
+// window cotangents (60 values per cell and direction) never leave the SM:
+// writing and gathering them through memory was 126 + 126 MB per direction at
+// 64^3, two thirds of the VJP's time. gw: 15 blocks of n, the x, y, z parts.
+//
+// k_adj_reduce: adds the parts and the second viscous part to a cell's
+// cotangent and goes on, in the same thread, with what is pointwise after it:
+// the end of a step (finish) and the next stage's adjoint.
+// ---------------------------------------------------------------------------
+constexpr int ADJ_T = 128;
+constexpr int ADJ_NC = 300;  // cells of a block's lines, at most (48 KB of shared memory)
+
+template <int RC>
+constexpr int adj_smem(int nc) { return nc * (RC == RC_WENO5 ? 20 : 5) * (int)sizeof(double); }
+
+template <int DIR, int FVS, int RC>
+__device__ __forceinline__ void adj_lines(const DevParams& P, const StateView& W,
+                                          const double* __restrict__ lamR, double* __restrict__ out,
+                                          int b, int lb, double* sm) {
+    constexpr int S = Stencil<RC>::S;
+    constexpr int MID = (S - 1) / 2;
+    const long long n = P.n;
+    const LineTile<DIR> tl(P, b, lb);
+    const int nc = tl.nc;
+    const double inv_h = DIR == 0 ? P.inv_dx : (DIR == 1 ? P.inv_dy : P.inv_dz);
+    // cotangent of the face between positions s and s+1, component q
+    auto lam_face = [&](int l, int s, int q) {
+        return inv_h * (lamR[q * n + tl.id(l, s + 1 == tl.len ? 0 : s + 1)] - lamR[q * n + tl.id(l, s)]);
+    };
+    auto split_jacobian = [&](int c, const double* gp, const double* gm) {
+        int l, s;
+        tl.of_slot(c, l, s);
+        const long long id = tl.id(l, s);
+        double w5[5], gw[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        load_w5(W, id, w5);
+        split_vjp<FVS, DIR>(w5, P.gamma, P.sw_eps, gp, gm, gw);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) out[q * n + id] = gw[q];
+    };
+    if constexpr (RC == RC_WENO5) {
+        double* F = sm;            // [10][nc]: F+0..4, F-0..4; then the cells' sums
+        double* G = sm + 10 * nc;  // [10][nc]: window cotangents of one component, plus then minus
+        for (int c = threadIdx.x; c < nc; c += ADJ_T) {
+            int l, s;
+            tl.of_slot(c, l, s);
+            double w5[5], Fp[5], Fm[5];
+            load_w5(W, tl.id(l, s), w5);
+            split_fwd<FVS, DIR>(w5, P, Fp, Fm);
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                F[q * nc + c] = Fp[q];
+                F[(5 + q) * nc + c] = Fm[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int q = 0; q < 5; ++q) {
+            for (int c = threadIdx.x; c < nc; c += ADJ_T) {
+                int l, s;
+                tl.of_slot(c, l, s);
+                const double lam = lam_face(l, s, q);
+                const double* fp = F + q * nc + l * tl.cl;
+                const double* fm = fp + 5 * nc;
+                double a[5], bm[5], ga[5] = {0, 0, 0, 0, 0}, gb[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    a[m] = fp[tl.at(s - MID + m)];
+                    bm[m] = fm[tl.at(s - MID + S - 1 - m)];
+                }
+                weno5_vjp(a, lam, ga);
+                weno5_vjp(bm, lam, gb);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    G[m * nc + c] = ga[m];
+                    G[(5 + m) * nc + c] = gb[m];
+                }
+            }
+            __syncthreads();
+            for (int c = threadIdx.x; c < nc; c += ADJ_T) {
+                int l, s;
+                tl.of_slot(c, l, s);
+                const double* g = G + l * tl.cl;
+                double sp = 0.0, sq = 0.0;
+#pragma unroll
+                for (int m = 0; m < 5; ++m) {
+                    // cell s = f - MID + m in the plus window of face f = s + MID - m,
+                    // and f - MID + (S-1-m) in the minus window of f = s + MID - S + 1 + m
+                    sp += g[m * nc + tl.at(s + MID - m)];
+                    sq += g[(5 + m) * nc + tl.at(s + MID - S + 1 + m)];
+                }
+                F[q * nc + c] = sp;  // component q's split fluxes are not read again
+                F[(5 + q) * nc + c] = sq;
+            }
+            __syncthreads();
+        }
+        for (int c = threadIdx.x; c < nc; c += ADJ_T) {
+            double gp[5], gm[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                gp[q] = F[q * nc + c];
+                gm[q] = F[(5 + q) * nc + c];
+            }
+            split_jacobian(c, gp, gm);
+        }
+    } else {
+        // a linear scheme's window cotangents are its coefficients times the face's
+        double* lf = sm;  // [5][nc]
+        for (int t = threadIdx.x; t < 5 * nc; t += ADJ_T) {
+            const int q = t / nc;
+            int l, s;
+            tl.of_slot(t - q * nc, l, s);
+            lf[t] = lam_face(l, s, q);
+        }
+        __syncthreads();
+        for (int c = threadIdx.x; c < nc; c += ADJ_T) {
+            int l, s;
+            tl.of_slot(c, l, s);
+            double gp[5], gm[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                const double* f = lf + q * nc + l * tl.cl;
+                double sp = 0.0, sq = 0.0;
+#pragma unroll
+                for (int m = 0; m < S; ++m) {
+                    const double c_m = RC == RC_LINEAR ? (m == 0 ? 1.0 : 0.0) : P.lin[m];
+                    sp += c_m * f[tl.at(s + MID - m)];
+                    sq += c_m * f[tl.at(s + MID - S + 1 + m)];
+                }
+                gp[q] = sp;
+                gm[q] = sq;
+            }
+            split_jacobian(c, gp, gm);
+        }
+    }
+}
+
+template <int FVS, int RC>
+__global__ void __launch_bounds__(ADJ_T, 4)
+k_adj_flux(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ gw,
+           double* __restrict__ lg, SmallShape sh) {
+    extern __shared__ double adj_sm[];
+    const long long n = P.n;
+    int b = blockIdx.x;
+    if (b < sh.nb[0]) { adj_lines<0, FVS, RC>(P, W, lamR, gw, b, sh.lb[0], adj_sm); return; }
+    b -= sh.nb[0];
+    if (b < sh.nb[1]) { adj_lines<1, FVS, RC>(P, W, lamR, gw + 5 * n, b, sh.lb[1], adj_sm); return; }
+    b -= sh.nb[1];
+    if (b < sh.nb[2]) { adj_lines<2, FVS, RC>(P, W, lamR, gw + 10 * n, b, sh.lb[2], adj_sm); return; }
+    b -= sh.nb[2];
+    const long long c = (long long)b * ADJ_T + threadIdx.x;
+    if (c >= n) return;
+    const int i = (int)(c % P.nx), j = (int)(c / P.nx % P.ny), k = (int)(c / ((long long)P.nx * P.ny));
+    if (P.vis_order == 4) adj_visc1_cell<4>(P, W, lamR, lg, i, j, k);
+    else if (P.vis_order == 6) adj_visc1_cell<6>(P, W, lamR, lg, i, j, k);
+    else adj_visc1_cell<8>(P, W, lamR, lg, i, j, k);
 }
 
 // Adjoint of one stage. Wk: the stage's output state, Wp: its input state.
 // Stage coefficients (U_k = a U0 + bU U(Wp) + bR dt R(Wp)): (1, 0, 1),
 // (3/4, 1/4, 1/4), (1/3, 2/3, 2/3). Writes lamR, initialises lamWp with the
 // U(Wp) part and accumulates lamU0 (set at stage 3, the first one reversed).
-template <int STAGE>
-__global__ void __launch_bounds__(256)
-k_adj_stage(DevParams P, StateView Wk, StateView Wp, const double* __restrict__ lamWk,
-            double* __restrict__ lamU0, double* __restrict__ lamR, double* __restrict__ lamWp,
-            double dt) {
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= P.n) return;
+__device__ __forceinline__ void adj_stage_cell(const DevParams& P, int stage, const double wk[5],
+                                               const StateView& Wp, long long id, const double lw[5],
+                                               double* __restrict__ lamU0, double* __restrict__ lamR,
+                                               double* __restrict__ lamWp, double dt) {
     const long long n = P.n;
-    const double a = STAGE == 1 ? 1.0 : (STAGE == 2 ? 0.75 : 1.0 / 3.0);
-    const double bU = STAGE == 1 ? 0.0 : (STAGE == 2 ? 0.25 : 2.0 / 3.0);
-    const double bR = STAGE == 1 ? 1.0 : bU;
-    double wk[5], lw[5], lU[5];
-    load_w5(Wk, id, wk);
-#pragma unroll
-    for (int q = 0; q < 5; ++q) lw[q] = lamWk[q * n + id];
+    const double a = stage == 1 ? 1.0 : (stage == 2 ? 0.75 : 1.0 / 3.0);
+    const double bU = stage == 1 ? 0.0 : (stage == 2 ? 0.25 : 2.0 / 3.0);
+    const double bR = stage == 1 ? 1.0 : bU;
+    double lU[5];
     c2p_vjp(wk, P.gamma, lw, lU);
     double lp[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (STAGE != 1) {
+    if (stage != 1) {
         double wp[5], lUp[5];
         load_w5(Wp, id, wp);
 #pragma unroll
@@ -313,26 +469,66 @@ k_adj_stage(DevParams P, StateView Wk, StateView Wp, const double* __restrict__ 
     }
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-        if (STAGE == 3) lamU0[q * n + id] = a * lU[q];
+        if (stage == 3) lamU0[q * n + id] = a * lU[q];
         else lamU0[q * n + id] += a * lU[q];
         lamR[q * n + id] = bR * dt * lU[q];
         lamWp[q * n + id] = lp[q];
     }
 }
 
-// lamW0 += (dU0/dW0)^T lamU0 (U0 = primitiveToConserved of the step's start).
+// One stage reversed at the end of a segment (in the middle, k_adj_reduce).
 __global__ void __launch_bounds__(256)
-k_adj_finish(DevParams P, StateView W0, const double* __restrict__ lamU0, double* __restrict__ lamW0) {
+k_adj_stage(DevParams P, int stage, StateView Wk, StateView Wp, const double* lamWk,
+            double* __restrict__ lamU0, double* __restrict__ lamR, double* lamWp, double dt) {
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= P.n) return;
+    double wk[5], lw[5];
+    load_w5(Wk, id, wk);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) lw[q] = lamWk[q * P.n + id];
+    adj_stage_cell(P, stage, wk, Wp, id, lw, lamU0, lamR, lamWp, dt);
+}
+
+// lamW (the cotangent of state W so far) += the parts of k_adj_flux; finish:
+// lamW += (dU0/dW)^T lamU0 (W is a step's start state); next > 0: that stage's
+// adjoint, whose output state is W and whose input state is Wp, in place.
+template <int ORD>
+__global__ void __launch_bounds__(128)
+k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const double* __restrict__ lg,
+             double* lamW, int finish, int next, StateView Wp, double* __restrict__ lamU0,
+             double* __restrict__ lamR, double dt) {
     const long long n = P.n;
-    double w0[5], lU[5], lw[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    load_w5(W0, id, w0);
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= n) return;
+    const int i = (int)(id % P.nx), j = (int)(id / P.nx % P.ny), k = (int)(id / ((long long)P.nx * P.ny));
+    double lw[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) lU[q] = lamU0[q * n + id];
-    p2c_vjp(w0, P.gamma, lU, lw);
+    for (int q = 0; q < 5; ++q)
+        lw[q] = ((lamW[q * n + id] + gw[q * n + id]) + gw[(5 + q) * n + id]) + gw[(10 + q) * n + id];
+    adj_visc2_cell<ORD>(P, W, lg, i, j, k, lw);
+    double w5[5];
+    if (finish || next) load_w5(W, id, w5);
+    if (finish) {
+        double lU[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) lamW0[q * n + id] += lw[q];
+        for (int q = 0; q < 5; ++q) lU[q] = lamU0[q * n + id];
+        p2c_vjp(w5, P.gamma, lU, lw);
+    }
+    if (next) {
+        adj_stage_cell(P, next, w5, Wp, id, lw, lamU0, lamR, lamW, dt);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) lamW[q * n + id] = lw[q];
+    }
+}
+
+// The second viscous part alone, after the marching face kernels.
+template <int ORD>
+__global__ void __launch_bounds__(128)
+k_adj_visc1(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ lg) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.nx) return;
+    adj_visc1_cell<ORD>(P, W, lamR, lg, i, blockIdx.y, blockIdx.z);
 }
 
 // d/dW of J = sum 0.5 rho |u|^2 dV (compute_total_energy, postprocess.cpp:103).
@@ -349,8 +545,11 @@ k_adj_seed_ke(DevParams P, StateView W, double* __restrict__ lamW, double dV) {
     lamW[4 * n + id] = 0.0;
 }
 
+// Boxes with a line too long for a block of k_adj_flux: the marching kernels.
+bool long_lines(const DevParams& P) { return P.nx > ADJ_NC || P.ny > ADJ_NC || P.nz > ADJ_NC; }
+
 template <int DIR, int FVS, int RC>
-cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* lamW) {
+cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw) {
     const DevParams& P = L.P;
     const int ext = DIR == 0 ? P.ny : P.nx;
     const int other = DIR == 2 ? P.ny : P.nz;
@@ -364,27 +563,41 @@ cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double*
     const int cext = DIR == 0 ? P.ny : P.nx;
     const int tc = detail::threads_for(cext);
     const dim3 cg((cext + tc - 1) / tc, DIR == 0 ? P.nx : P.ny, P.nz);
-    k_adj_cell<DIR, FVS, RC><<<cg, tc, 0, L.stream>>>(P, W, G, lamW);
+    k_adj_cell<DIR, FVS, RC><<<cg, tc, 0, L.stream>>>(P, W, G, gw + 5 * DIR * P.n);
     return cudaGetLastError();
 }
 
+// G (long lines only): the window cotangents, 10 S blocks of n.
 template <int FVS, int RC>
-cudaError_t adj_inviscid(const LaunchCfg& L, StateView W, const double* lamR, double* G,
-                         double* lamW) {
-    cudaError_t e = adj_dir<0, FVS, RC>(L, W, lamR, G, lamW);
-    if (e == cudaSuccess) e = adj_dir<1, FVS, RC>(L, W, lamR, G, lamW);
-    if (e == cudaSuccess) e = adj_dir<2, FVS, RC>(L, W, lamR, G, lamW);
-    return e;
+cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw, double* lg) {
+    const DevParams& P = L.P;
+    if (!long_lines(P)) {
+        // 128 to 256 cells a block: several blocks per SM, at least two per SM for each direction
+        const long long target = std::min(256ll, std::max(64ll, 3 * P.n / (2 * 148)));
+        const SmallShape sh = small_shape(P, target, ADJ_NC, ADJ_T);
+        k_adj_flux<FVS, RC><<<small_blocks(sh), ADJ_T, adj_smem<RC>(small_cells(P, sh)), L.stream>>>(P, W, lamR, gw,
+                                                                                                   lg, sh);
+        return cudaGetLastError();
+    }
+    cudaError_t e = adj_dir<0, FVS, RC>(L, W, lamR, G, gw);
+    if (e == cudaSuccess) e = adj_dir<1, FVS, RC>(L, W, lamR, G, gw);
+    if (e == cudaSuccess) e = adj_dir<2, FVS, RC>(L, W, lamR, G, gw);
+    if (e != cudaSuccess) return e;
+    const int th = detail::threads_for(P.nx);
+    const dim3 g = detail::cell_grid(P, th);
+    if (P.vis_order == 4) k_adj_visc1<4><<<g, th, 0, L.stream>>>(P, W, lamR, lg);
+    else if (P.vis_order == 6) k_adj_visc1<6><<<g, th, 0, L.stream>>>(P, W, lamR, lg);
+    else k_adj_visc1<8><<<g, th, 0, L.stream>>>(P, W, lamR, lg);
+    return cudaGetLastError();
 }
 
 template <int FVS>
-cudaError_t adj_inviscid_rc(const LaunchCfg& L, StateView W, const double* lamR, double* G,
-                            double* lamW) {
+cudaError_t adj_flux_rc(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw, double* lg) {
     switch (L.rc) {
-    case RC_WENO5: return adj_inviscid<FVS, RC_WENO5>(L, W, lamR, G, lamW);
-    case RC_LINEAR: return adj_inviscid<FVS, RC_LINEAR>(L, W, lamR, G, lamW);
-    case RC_LIN6: return adj_inviscid<FVS, RC_LIN6>(L, W, lamR, G, lamW);
-    case RC_LIN8: return adj_inviscid<FVS, RC_LIN8>(L, W, lamR, G, lamW);
+    case RC_WENO5: return adj_flux<FVS, RC_WENO5>(L, W, lamR, G, gw, lg);
+    case RC_LINEAR: return adj_flux<FVS, RC_LINEAR>(L, W, lamR, G, gw, lg);
+    case RC_LIN6: return adj_flux<FVS, RC_LIN6>(L, W, lamR, G, gw, lg);
+    case RC_LIN8: return adj_flux<FVS, RC_LIN8>(L, W, lamR, G, gw, lg);
     default: return cudaErrorNotSupported;
     }
 }
@@ -392,45 +605,34 @@ cudaError_t adj_inviscid_rc(const LaunchCfg& L, StateView W, const double* lamR,
 }  // namespace
 
 int adj_scratch_blocks(const LaunchCfg& L) {
+    if (!long_lines(L.P)) return 15;
     const int S = L.rc == RC_LIN8 ? 8 : (L.rc == RC_LINEAR ? 2 : 6);
-    return 2 * S * 5;
+    return 15 + 2 * S * 5;
 }
 
-cudaError_t adj_rhs_vjp(const LaunchCfg& L, StateView W, const double* lamR, double* G,
-                        double* lg, double* lamW) {
-    cudaError_t e = L.fvs == FV_SW ? adj_inviscid_rc<FV_SW>(L, W, lamR, G, lamW)
-                                   : adj_inviscid_rc<FV_LF>(L, W, lamR, G, lamW);
+int adj_rhs_vjp_launches(const LaunchCfg& L) { return long_lines(L.P) ? 8 : 2; }
+
+cudaError_t adj_rhs_vjp(const LaunchCfg& L, StateView W, double* G, double* lg, double* lamW, int finish, int next,
+                        StateView Wp, double* lamU0, double* lamR, double dt) {
+    const DevParams& P = L.P;
+    double* gw = G;
+    double* Gw = G + 15 * P.n;
+    cudaError_t e = L.fvs == FV_SW ? adj_flux_rc<FV_SW>(L, W, lamR, Gw, gw, lg)
+                                   : adj_flux_rc<FV_LF>(L, W, lamR, Gw, gw, lg);
     if (e != cudaSuccess) return e;
-    const int th = detail::threads_for(L.P.nx);
-    const dim3 g = detail::cell_grid(L.P, th);
-    switch (L.P.vis_order) {
-    case 4:
-        k_adj_visc1<4><<<g, th, 0, L.stream>>>(L.P, W, lamR, lg);
-        k_adj_visc2<4><<<g, th, 0, L.stream>>>(L.P, W, lg, lamW);
-        break;
-    case 6:
-        k_adj_visc1<6><<<g, th, 0, L.stream>>>(L.P, W, lamR, lg);
-        k_adj_visc2<6><<<g, th, 0, L.stream>>>(L.P, W, lg, lamW);
-        break;
-    default:
-        k_adj_visc1<8><<<g, th, 0, L.stream>>>(L.P, W, lamR, lg);
-        k_adj_visc2<8><<<g, th, 0, L.stream>>>(L.P, W, lg, lamW);
-        break;
+    const unsigned b = (unsigned)((P.n + 127) / 128);
+    switch (P.vis_order) {
+    case 4: k_adj_reduce<4><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
+    case 6: k_adj_reduce<6><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
+    default: k_adj_reduce<8><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
     }
     return cudaGetLastError();
 }
 
-cudaError_t adj_stage(const LaunchCfg& L, int stage, StateView Wk, StateView Wp,
-                      const double* lamWk, double* lamU0, double* lamR, double* lamWp, double dt) {
-    const unsigned b = (unsigned)((L.P.n + 255) / 256);
-    if (stage == 1) k_adj_stage<1><<<b, 256, 0, L.stream>>>(L.P, Wk, Wp, lamWk, lamU0, lamR, lamWp, dt);
-    else if (stage == 2) k_adj_stage<2><<<b, 256, 0, L.stream>>>(L.P, Wk, Wp, lamWk, lamU0, lamR, lamWp, dt);
-    else k_adj_stage<3><<<b, 256, 0, L.stream>>>(L.P, Wk, Wp, lamWk, lamU0, lamR, lamWp, dt);
-    return cudaGetLastError();
-}
-
-cudaError_t adj_finish(const LaunchCfg& L, StateView W0, const double* lamU0, double* lamW0) {
-    k_adj_finish<<<(unsigned)((L.P.n + 255) / 256), 256, 0, L.stream>>>(L.P, W0, lamU0, lamW0);
+cudaError_t adj_stage(const LaunchCfg& L, int stage, StateView Wk, StateView Wp, const double* lamWk, double* lamU0,
+                      double* lamR, double* lamWp, double dt) {
+    k_adj_stage<<<(unsigned)((L.P.n + 255) / 256), 256, 0, L.stream>>>(L.P, stage, Wk, Wp, lamWk, lamU0, lamR, lamWp,
+                                                                       dt);
     return cudaGetLastError();
 }
 

@@ -85,8 +85,8 @@ struct ns3d_ctx {
     double* step_times = nullptr;  // current_time after each step of the last run call
     // device scratch of the adjoint entry points, kept between calls (grown,
     // never shrunk; freed with the context)
-    double* adj_buf[10] = {};
-    size_t adj_cap[10] = {};
+    double* adj_buf[9] = {};
+    size_t adj_cap[9] = {};
     int step_times_cap = 0, step_times_n = 0;
     double time = 0.0, out_next = 0.0;
     long long steps = 0;         // completed steps (the time_advance step count beside `time`)
@@ -1501,7 +1501,7 @@ struct DevBuf {
 };
 
 // The adjoint's scratch arrays, by role.
-enum { AB_CK, AB_WS, AB_LA, AB_LB, AB_LU0, AB_LR, AB_G, AB_LG, AB_DTD, AB_LW, AB_COUNT };
+enum { AB_CK, AB_WS, AB_LA, AB_LU0, AB_LR, AB_G, AB_LG, AB_DTD, AB_LW, AB_COUNT };
 
 // `count` doubles of adjoint scratch `slot`, kept in the context: a call that
 // needs no more than an earlier one allocates nothing (allocating and freeing
@@ -1553,7 +1553,8 @@ ns3d_status ns3d_rhs_vjp(ns3d_ctx* ctx, const double* lam_rhs, double* lam_w) {
     if (!lr || !lw || !G || !lg) return fail(ctx, NS3D_ERR_NOMEM, "adjoint scratch allocation failed");
     NS3D_CK(cudaMemcpyAsync(lr, lam_rhs, sizeof(double) * 5 * n, cudaMemcpyHostToDevice, ctx->stream));
     NS3D_CK(cudaMemsetAsync(lw, 0, sizeof(double) * 5 * n, ctx->stream));
-    NS3D_LAUNCH(NS3D_KERNEL_OTHER, 11, adj_rhs_vjp(ctx->L, view(ctx, ctx->cur), lr, G, lg, lw));
+    NS3D_LAUNCH(NS3D_KERNEL_OTHER, adj_rhs_vjp_launches(ctx->L),
+                adj_rhs_vjp(ctx->L, view(ctx, ctx->cur), G, lg, lw, 0, 0, StateView{}, nullptr, lr, 0.0));
     NS3D_CK(cudaMemcpyAsync(lam_w, lw, sizeof(double) * 5 * n, cudaMemcpyDeviceToHost, ctx->stream));
     NS3D_CK(cudaStreamSynchronize(ctx->stream));
     return NS3D_OK;
@@ -1584,41 +1585,65 @@ ns3d_status ns3d_adjoint(ns3d_ctx* ctx, int nsteps, int K, const double* dts_in,
     const long long n = ctx->n;
     const size_t st = 6 * (size_t)n;  // one state: rho,u,v,w,p,T
     const int nseg = (nsteps + K - 1) / K;
-    double* ck = adj_scratch(ctx, AB_CK, st * nseg);
+    double* ck = nseg > 1 ? adj_scratch(ctx, AB_CK, st * (nseg - 1)) : nullptr;
     double* ws = adj_scratch(ctx, AB_WS, st * (3 * (size_t)K + 1));
     double* la = adj_scratch(ctx, AB_LA, 5 * n);
-    double* lb = adj_scratch(ctx, AB_LB, 5 * n);
     double* lu0 = adj_scratch(ctx, AB_LU0, 5 * n);
     double* lr = adj_scratch(ctx, AB_LR, 5 * n);
     double* G = adj_scratch(ctx, AB_G, (size_t)adj_scratch_blocks(ctx->L) * n);
     double* lg = adj_scratch(ctx, AB_LG, 16 * n);
     double* dtd = adj_scratch(ctx, AB_DTD, nsteps);
-    if (!ck || !ws || !la || !lb || !lu0 || !lr || !G || !lg || !dtd)
+    if ((nseg > 1 && !ck) || !ws || !la || !lu0 || !lr || !G || !lg || !dtd)
         return fail(ctx, NS3D_ERR_NOMEM, "adjoint checkpoint/scratch allocation failed");
     std::vector<double> dts(nsteps);
 
-    // ---- forward run, a checkpoint every K steps, dt recorded ----
+    // stage states of a segment: state(j, stg) is the output of stage stg of
+    // its step j, state(j, 0) that step's start
+    auto state_ptr = [&](int j, int stg) { return ws + (size_t)(3 * j + stg) * st; };
+    auto state = [&](int j, int stg) { return view_at(state_ptr(j, stg), n); };
+    auto segment_step = [&](int j) -> ns3d_status {
+        for (int stg = 1; stg <= 3; ++stg) {
+            const ns3d_status e = stage_at(ctx, stg, state_ptr(j, stg - 1), state_ptr(j, 0), state_ptr(j, stg));
+            if (e != NS3D_OK) return e;
+        }
+        return NS3D_OK;
+    };
+
+    // ---- forward run, a checkpoint every K steps, dt recorded; the last
+    // segment's steps leave their stage states where the reverse sweep, which
+    // begins with them, needs them ----
     if ((s = reset_ctrl(ctx)) != NS3D_OK) return s;
+    const int last0 = (nseg - 1) * K, cur0 = ctx->cur;
     for (int k = 0; k < nsteps; ++k) {
+        const bool kept = k >= last0;
         if (k % K == 0)
-            NS3D_CK(cudaMemcpyAsync(ck + (size_t)(k / K) * st, warr(ctx, ctx->cur, 0),
+            NS3D_CK(cudaMemcpyAsync(kept ? ws : ck + (size_t)(k / K) * st, warr(ctx, ctx->cur, 0),
                                     sizeof(double) * st, cudaMemcpyDeviceToDevice, ctx->stream));
-        ctx->rec = ctx->cur;
+        const StateView W = kept ? state(k - last0, 0) : view(ctx, ctx->cur);
+        if (!kept) ctx->rec = ctx->cur;
         if (dts_in) {
             if ((s = set_dt(ctx, dts_in[k])) != NS3D_OK) return s;
         } else {
             std::memcpy(&ctx->ctrl_host->dtmin_bits, &CFL_INIT, sizeof(double));
             NS3D_CK(cudaMemcpyAsync(&ctx->ctrl->dtmin_bits, &ctx->ctrl_host->dtmin_bits,
                                     sizeof(unsigned long long), cudaMemcpyHostToDevice, ctx->stream));
-            if ((s = enqueue_cfl(ctx)) != NS3D_OK) return s;
+            NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
+                        (k_cfl<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(ctx->L.P, W, ctx->ctrl)));
             NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1,
                         launch_pdl(ctx->L, k_control, 1, 1, 0, ctx->ctrl, (int)CONTROL_PRE, 0, ctx->p.cfl,
                                    ctx->p.dt_fixed, 0.0, 0.0, n, (double*)nullptr));
         }
         NS3D_CK(cudaMemcpyAsync(dtd + k, &ctx->ctrl->dt, sizeof(double), cudaMemcpyDeviceToDevice,
                                 ctx->stream));
-        if ((s = enqueue_rk3(ctx)) != NS3D_OK) return s;
+        if ((s = kept ? segment_step(k - last0) : enqueue_rk3(ctx)) != NS3D_OK) return s;
     }
+    // the context's buffers as that many enqueue_rk3 calls leave them
+    ctx->cur = (cur0 + nsteps) % 3;
+    ctx->rec = (cur0 + nsteps - 1) % 3;
+    NS3D_CK(cudaMemcpyAsync(warr(ctx, ctx->rec, 0), state_ptr(nsteps - 1 - last0, 0), sizeof(double) * st,
+                            cudaMemcpyDeviceToDevice, ctx->stream));
+    NS3D_CK(cudaMemcpyAsync(warr(ctx, ctx->cur, 0), state_ptr(nsteps - 1 - last0, 3), sizeof(double) * st,
+                            cudaMemcpyDeviceToDevice, ctx->stream));
     NS3D_CK(cudaMemcpyAsync(dts.data(), dtd, sizeof(double) * nsteps, cudaMemcpyDeviceToHost,
                             ctx->stream));
     if ((s = read_ctrl(ctx)) != NS3D_OK) return s;
@@ -1631,7 +1656,6 @@ ns3d_status ns3d_adjoint(ns3d_ctx* ctx, int nsteps, int K, const double* dts_in,
 
     // ---- seed: dJ/dw at the end state ----
     double* A = la;
-    double* B = lb;
     if (lam_final)
         NS3D_CK(cudaMemcpyAsync(A, lam_final, sizeof(double) * 5 * n, cudaMemcpyHostToDevice, ctx->stream));
     else
@@ -1641,27 +1665,26 @@ ns3d_status ns3d_adjoint(ns3d_ctx* ctx, int nsteps, int K, const double* dts_in,
     // ---- reverse sweep, segment by segment ----
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int s0 = seg * K, m = std::min(K, nsteps - s0);
-        NS3D_CK(cudaMemcpyAsync(ws, ck + (size_t)seg * st, sizeof(double) * st,
-                                cudaMemcpyDeviceToDevice, ctx->stream));
-        for (int j = 0; j < m; ++j) {  // recompute the segment's stage states
-            double* w0 = ws + (size_t)(3 * j) * st;
-            if ((s = set_dt(ctx, dts[s0 + j])) != NS3D_OK) return s;
-            if ((s = stage_at(ctx, 1, w0, w0, w0 + st)) != NS3D_OK) return s;
-            if ((s = stage_at(ctx, 2, w0 + st, w0, w0 + 2 * st)) != NS3D_OK) return s;
-            if ((s = stage_at(ctx, 3, w0 + 2 * st, w0, w0 + 3 * st)) != NS3D_OK) return s;
-        }
-        for (int j = m - 1; j >= 0; --j) {  // A: adjoint of the step's end state
-            double* w0 = ws + (size_t)(3 * j) * st;
-            const double dt = dts[s0 + j];
-            for (int stg = 3; stg >= 1; --stg) {
-                const StateView Wk = view_at(w0 + (size_t)stg * st, n);
-                const StateView Wp = view_at(w0 + (size_t)(stg - 1) * st, n);
-                NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1, adj_stage(ctx->L, stg, Wk, Wp, A, lu0, lr, B, dt));
-                NS3D_LAUNCH(NS3D_KERNEL_OTHER, 11, adj_rhs_vjp(ctx->L, Wp, lr, G, lg, B));
-                std::swap(A, B);
+        if (seg < nseg - 1) {  // recompute the segment's stage states
+            NS3D_CK(cudaMemcpyAsync(ws, ck + (size_t)seg * st, sizeof(double) * st,
+                                    cudaMemcpyDeviceToDevice, ctx->stream));
+            for (int j = 0; j < m; ++j) {
+                if ((s = set_dt(ctx, dts[s0 + j])) != NS3D_OK) return s;
+                if ((s = segment_step(j)) != NS3D_OK) return s;
             }
-            NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1, adj_finish(ctx->L, view_at(w0, n), lu0, A));
         }
+        // A: cotangent of the segment's end state, then of every stage's input
+        // state, the reverse of each following stage fused with the reduction
+        NS3D_LAUNCH(NS3D_KERNEL_OTHER, 1, adj_stage(ctx->L, 3, state(m - 1, 3), state(m - 1, 2), A, lu0, lr, A,
+                                                    dts[s0 + m - 1]));
+        for (int j = m - 1; j >= 0; --j)
+            for (int stg = 3; stg >= 1; --stg) {
+                const int finish = stg == 1, next = stg > 1 ? stg - 1 : (j > 0 ? 3 : 0);
+                const StateView Wp = next == 0 ? StateView{} : (stg > 1 ? state(j, stg - 2) : state(j - 1, 2));
+                const double dt = dts[s0 + (stg > 1 ? j : std::max(j - 1, 0))];
+                NS3D_LAUNCH(NS3D_KERNEL_OTHER, adj_rhs_vjp_launches(ctx->L),
+                            adj_rhs_vjp(ctx->L, state(j, stg - 1), G, lg, A, finish, next, Wp, lu0, lr, dt));
+            }
     }
     NS3D_CK(cudaMemcpyAsync(grad, A, sizeof(double) * 5 * n, cudaMemcpyDeviceToHost, ctx->stream));
     NS3D_CK(cudaStreamSynchronize(ctx->stream));

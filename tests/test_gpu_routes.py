@@ -132,6 +132,59 @@ def test_noalloc_captured_in_a_graph():
     assert torch.equal(rhs, want) and bool(torch.isfinite(rhs).all())
 
 
+# k_adj_flux (every extent at most 300) and the marching adjoint kernels, with
+# a partial last group of lines and the last extent each side of the limit
+@pytest.mark.parametrize("kw", [dict(sw_entropy_eps=1e-3), dict(fvs_type="LaxFriedrichs", recon="MDCD"),
+                                dict(recon="UD7L", vis_scheme="C6th"), dict(recon="LINEAR", vis_scheme="C4th")],
+                         ids=scheme_id)
+@pytest.mark.parametrize("box", [(10, 9, 8), (33, 12, 8), (300, 8, 8), (8, 301, 8), (9, 8, 304)],
+                         ids=lambda b: "x".join(map(str, b)))
+def test_rhs_vjp_routes_dot_product(box, kw):
+    """<lam, dR[v]> by 4-point central differences equals <R^T lam, v> (the
+    1e-7 of the cubic box's test, of the product's largest possible value)."""
+    p = _box_params(box, **kw)
+    nx, ny, nz = box
+    Z, Y, X = np.meshgrid(*[np.arange(m) * (2 * np.pi / m) for m in (nz, ny, nx)], indexing="ij")
+    W = np.stack([1 + 0.1 * np.sin(X + 0.3) * np.cos(Y + Z), 0.5 + 0.2 * np.sin(X) * np.cos(Y) * np.cos(Z),
+                  0.4 - 0.2 * np.cos(X) * np.sin(Y) * np.cos(Z), 0.6 + 0.1 * np.sin(Z + X),
+                  7.9 + 0.5 * np.cos(2 * X) * np.cos(Y + Z)])
+    rng = np.random.default_rng(4)
+    lam, v = rng.standard_normal(W.shape), np.stack([0.01 * np.sin(X + 2 * Y), np.cos(Y - Z), np.sin(Z + X),
+                                                     np.cos(X + Y + Z), 0.3 * np.sin(2 * Z - X)])
+    h, r = 1e-5, {}
+    with ns.Solver(p) as s:
+        for k in (-2, -1, 1, 2):
+            s.upload_primitive(W + k * h * v)
+            r[k] = s.compute_rhs()
+        s.upload_primitive(W)
+        g = s.rhs_vjp(lam)
+    fd = float(np.sum(lam * (-r[2] + 8 * r[1] - 8 * r[-1] + r[-2])) / (12 * h))
+    ad = float(np.sum(g * v))
+    assert abs(fd - ad) <= 1e-7 * np.linalg.norm(g) * np.linalg.norm(v), (fd, ad)
+
+
+def test_adjoint_leaves_end_state_and_recorded_state():
+    """After ns3d_adjoint the context holds the end state and the last step's
+    start as U0, whether the last segment is whole, partial or the only one."""
+    box, W = (16, 12, 10), _field((16, 12, 10))
+    p = _box_params(box, sw_entropy_eps=1e-3)
+    with ns.Solver(p) as s:
+        s.upload_primitive(W)
+        _, _, dts = s.adjoint(4, 2)
+        grads = []
+        for K in (1, 2, 3, 4, 9):
+            s.upload_primitive(W)
+            g, J, d = s.adjoint(4, K, dts=dts)
+            end, res = s.download_primitive(), s.residuals()
+            s.upload_primitive(W)
+            s.step_dts(dts)
+            assert np.array_equal(end, s.download_primitive())
+            assert np.array_equal(res, s.residuals())
+            grads.append(g)
+    for g in grads[1:]:
+        assert np.array_equal(g, grads[0])
+
+
 EXTREME = [("p", 1e160), ("p", np.inf), ("u", np.nan), ("u", 1e200), ("rho", 1e305),
            ("w", -np.inf), ("p", -1.0), ("p", 0.0)]
 
