@@ -92,8 +92,7 @@ inline int segment_for(int len, long long lines) {
 
 }  // namespace detail
 
-// Whether an FP64 box takes launch_flux_small: component-wise schemes, every
-// line short enough for a block's shared memory, no tuning override of the
+// Whether an FP64 box takes launch_flux_small: every line short enough for a block's shared memory, no tuning override of the
 // marching kernels, and few enough cells: L.small (1500000) where nx is a
 // multiple of 32 and the x sweep marches a warp per row (a step at 64^3 356 ->
 // 265 us, 112^3 1917 -> 1508 us WENO5 and 1214 -> 1044 us MDCD; 128^3 2092 -> 2102
@@ -102,8 +101,9 @@ inline int segment_for(int len, long long lines) {
 // larger ones not measured).
 inline bool small_box(const LaunchCfg& L) {
     const DevParams& P = L.P;
-    return L.small && !L.chr && P.n <= (P.nx % 32 == 0 ? L.small : 6 * L.small) && P.nx <= SMALL_NC &&
-           P.ny <= SMALL_NC && P.nz <= SMALL_NC;
+    const int most = small_most(L.chr != 0);
+    return L.small && P.n <= (P.nx % 32 == 0 && !L.chr ? L.small : 6 * L.small) && P.nx <= most && P.ny <= most &&
+           P.nz <= most;
 }
 
 // Boxes whose launches overlap by programmatic dependent launch: those whose
@@ -345,31 +345,35 @@ cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, doubl
 
 #ifdef NS3D_LAUNCH_SMALL
 namespace detail {
-template <int FVS, int RC>
+template <int FVS, int RC, bool CHR>
 cudaError_t flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
     // 64 to 256 cells a block, so that the three sweeps give at least two blocks per SM
     const long long target = std::min(256ll, std::max(64ll, 3 * L.P.n / (2 * 148)));
-    const SmallShape sh = small_shape(L.P, target, SMALL_NC, SMALL_T);
+    const SmallShape sh = small_shape(L.P, target, small_most(CHR), SMALL_T);
     const int nc = small_cells(L.P, sh);
     const unsigned blocks = small_blocks(sh);
-    return launch_pdl(L, k_flux_small<FVS, RC>, blocks, SMALL_T, small_smem(nc), L.P, W, tacc, fv, sh, ctrl);
+    return launch_pdl(L, k_flux_small<FVS, RC, CHR>, blocks, SMALL_T, small_smem(nc, CHR), L.P, W, tacc, fv, sh, ctrl);
 }
 }  // namespace detail
 
 cudaError_t launch_flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
-    auto by_rc = [&](auto fvs) -> cudaError_t {
+    auto by_rc = [&](auto fvs, auto chr) -> cudaError_t {
         constexpr int FVS = decltype(fvs)::value;
+        constexpr bool CHR = decltype(chr)::value;
         switch (L.rc) {
-        case RC_WENO5: return detail::flux_small<FVS, RC_WENO5>(L, W, tacc, fv, ctrl);
-        case RC_LINEAR: return detail::flux_small<FVS, RC_LINEAR>(L, W, tacc, fv, ctrl);
-        case RC_LIN6: return detail::flux_small<FVS, RC_LIN6>(L, W, tacc, fv, ctrl);
-        case RC_MDCD_HYBRID: return detail::flux_small<FVS, RC_MDCD_HYBRID>(L, W, tacc, fv, ctrl);
-        case RC_LIN8: return detail::flux_small<FVS, RC_LIN8>(L, W, tacc, fv, ctrl);
+        case RC_WENO5: return detail::flux_small<FVS, RC_WENO5, CHR>(L, W, tacc, fv, ctrl);
+        case RC_LINEAR: return detail::flux_small<FVS, RC_LINEAR, CHR>(L, W, tacc, fv, ctrl);
+        case RC_LIN6: return detail::flux_small<FVS, RC_LIN6, CHR>(L, W, tacc, fv, ctrl);
+        case RC_MDCD_HYBRID: return detail::flux_small<FVS, RC_MDCD_HYBRID, CHR>(L, W, tacc, fv, ctrl);
+        case RC_LIN8: return detail::flux_small<FVS, RC_LIN8, CHR>(L, W, tacc, fv, ctrl);
         default: return cudaErrorInvalidValue;
         }
     };
-    return L.fvs == FV_SW ? by_rc(std::integral_constant<int, FV_SW>{})
-                          : by_rc(std::integral_constant<int, FV_LF>{});
+    auto by_fvs = [&](auto chr) {
+        return L.fvs == FV_SW ? by_rc(std::integral_constant<int, FV_SW>{}, chr)
+                              : by_rc(std::integral_constant<int, FV_LF>{}, chr);
+    };
+    return L.chr ? by_fvs(std::true_type{}) : by_fvs(std::false_type{});
 }
 
 template <int ORD>

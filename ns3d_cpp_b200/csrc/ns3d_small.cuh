@@ -101,10 +101,111 @@ struct LineTile {
     __device__ __forceinline__ int at(int s) const { return wrap1(s, len) * cs; }
 };
 
-constexpr int small_smem(int nc) { return nc * 15 * (int)sizeof(double); }
+// Shared doubles per cell: split fluxes (10), faces (5) and, for the
+// characteristic-wise reconstruction, the Roe averages' terms (5); cells of a
+// block's lines at most.
+constexpr int small_doubles(bool chr) { return chr ? 20 : 15; }
+constexpr int small_most(bool chr) { return chr ? 300 : SMALL_NC; }
+constexpr int small_smem(int nc, bool chr) { return nc * small_doubles(chr) * (int)sizeof(double); }
+
+// char_face with everything by the general code, for faces whose values come
+// out infinite or NaN below.
+template <int DIR, int RC>
+__device__ __noinline__ void char_face_cold(const DevParams& P, const double* wl, const double* wr,
+                                            const double* F, int nc, const int* w, double* face) {
+    char_face<DIR, double, RC>(P.gamma, wl, wr, [&](int m, int r) { return F[r * nc + w[m]]; },
+                               [&](int m, int r) { return F[(5 + r) * nc + w[m]]; }, P.lin,
+                               P.mdcd_disp, P.mdcd_diss, face);
+}
+
+// The face of char_face from the split fluxes F ([10][nc]) at slots w and the
+// Roe terms g ([5][nc]: sqrt rho, u, v, w, H) of its two cells: the same
+// operations in the same order, without the products with the eigenvectors'
+// structural zeros and ones (each adds a zero or is the factor itself: 310
+// instead of 500 operations for the projections) and with the branch-free
+// quotients. One side's five projected windows are held at a time.
+template <int DIR, int RC>
+__device__ __forceinline__ void char_face_fast(const DevParams& P, const double* __restrict__ F,
+                                               const double* __restrict__ g, int nc, const int* w,
+                                               double face[5]) {
+    constexpr int S = Stencil<RC>::S;
+    constexpr int MID = (S - 1) / 2;
+    const double gm1 = P.gamma - 1.0;
+    const int cl = w[MID], cr = w[MID + 1];
+    const double sl = g[cl], sr = g[cr];
+    const double den = quot_mid(1.0, sl + sr);
+    auto avg = [&](int k) { return (sl * g[k * nc + cl] + sr * g[k * nc + cr]) * den; };
+    const double u0 = avg(1), v0 = avg(2), w0 = avg(3), h0 = avg(4);
+    const double V = 0.5 * (u0 * u0 + v0 * v0 + w0 * w0);
+    const double un = DIR == 0 ? u0 : (DIR == 1 ? v0 : w0);
+    const double c = sqrt_mid(gm1 * (h0 - V));
+    const double t2 = DIR == 0 ? v0 : (DIR == 1 ? w0 : u0);
+    const double t3 = DIR == 0 ? w0 : (DIR == 1 ? u0 : v0);
+    const double chi = quot_mid(0.5, c), K = quot_mid(gm1, c * c), K1 = 0.5 * K;
+    // rows 0, 1, 4 of the left eigenvectors; rows 2 and 3 are (-t2, unit vector)
+    // and (-t3, unit vector)
+    const double ku[3] = {K1 * u0, K1 * v0, K1 * w0};
+    double L0[5], L1[5], L4[5];
+    L0[0] = K1 * V + chi * un;
+    L4[0] = K1 * V - chi * un;
+    L1[0] = 1.0 - K * V;
+    L1[1] = K * u0; L1[2] = K * v0; L1[3] = K * w0; L1[4] = -K;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        L0[1 + d] = d == DIR ? -chi - ku[d] : -ku[d];
+        L4[1 + d] = d == DIR ? chi - ku[d] : -ku[d];
+    }
+    L0[4] = K1;
+    L4[4] = K1;
+    constexpr int E2 = DIR == 0 ? 2 : (DIR == 1 ? 3 : 1);  // the unit component of rows 2, 3
+    constexpr int E3 = DIR == 0 ? 3 : (DIR == 1 ? 1 : 2);
+    double wc[5];
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        double a[5][S];
+#pragma unroll
+        for (int m = 0; m < S; ++m) {
+            // reconstruct_select reverses the minus window; WENO5 reads five values
+            if (RC == RC_WENO5 && m == 5) continue;
+            const int sl_ = w[side == 0 ? m : S - 1 - m];
+            double f[5];
+#pragma unroll
+            for (int r = 0; r < 5; ++r) f[r] = F[(5 * side + r) * nc + sl_];
+            double s0 = L0[0] * f[0], s1 = L1[0] * f[0], s4 = L4[0] * f[0];
+#pragma unroll
+            for (int r = 1; r < 5; ++r) {
+                s0 += L0[r] * f[r];
+                s1 += L1[r] * f[r];
+                s4 += L4[r] * f[r];
+            }
+            a[0][m] = s0;
+            a[1][m] = s1;
+            a[2][m] = -t2 * f[0] + f[E2];
+            a[3][m] = -t3 * f[0] + f[E3];
+            a[4][m] = s4;
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const double r = reconstruct<double, RC>(a[q], P.lin, P.mdcd_disp, P.mdcd_diss);
+            wc[q] = side == 0 ? r : wc[q] + r;
+        }
+    }
+    // the right eigenvectors' rows on wc
+    const double uc = un * c, vel[3] = {u0, v0, w0};
+    face[0] = (wc[0] + wc[1]) + wc[4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double lo = d == DIR ? vel[d] - c : vel[d], hi = d == DIR ? vel[d] + c : vel[d];
+        double t = lo * wc[0] + vel[d] * wc[1];
+        if (1 + d == E2) t += wc[2];
+        if (1 + d == E3) t += wc[3];
+        face[1 + d] = t + hi * wc[4];
+    }
+    face[4] = (((h0 - uc) * wc[0] + V * wc[1]) + t2 * wc[2] + t3 * wc[3]) + (h0 + uc) * wc[4];
+}
 
 // The sweep along DIR of the lines of block b: out (5 blocks of n).
-template <int DIR, int FVS, int RC>
+template <int DIR, int FVS, int RC, bool CHR>
 __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView& W,
                                             double* __restrict__ out, int b, int lb, double* sm) {
     constexpr int S = Stencil<RC>::S;
@@ -114,6 +215,7 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
     const int nc = tl.nc;
     double* F = sm;             // [10][nc]: F+0..4, F-0..4
     double* fl = sm + 10 * nc;  // [5][nc]: face right of each cell
+    double* g = sm + 15 * nc;   // CHR [5][nc]: sqrt rho, u, v, w, H of each cell (roe_state)
     for (int c = threadIdx.x; c < nc; c += SMALL_T) {
         int l, s;
         tl.of_slot(c, l, s);
@@ -126,40 +228,75 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
             F[q * nc + c] = Fp[q];
             F[(5 + q) * nc + c] = Fm[q];
         }
+        if constexpr (CHR) {
+            const double rho = raw[0], p = raw[4];
+            const double E = rho * (0.5 * (raw[1] * raw[1] + raw[2] * raw[2] + raw[3] * raw[3]) +
+                                    quot_mid(p, (P.gamma - 1.0) * rho));
+            g[c] = sqrt_mid(rho);
+            g[nc + c] = raw[1];
+            g[2 * nc + c] = raw[2];
+            g[3 * nc + c] = raw[3];
+            g[4 * nc + c] = quot_mid(E + p, rho);
+        }
     }
     __syncthreads();
-    // a thread takes a face's components one after the other; of a block with no
-    // more cells than half its threads two threads share them
-    const bool two = nc <= SMALL_T / 2;
-    const int half = two && threadIdx.x >= SMALL_T / 2 ? 1 : 0;
-    const int q0 = half ? 3 : 0, q1 = two && !half ? 3 : 5;
-    for (int c = threadIdx.x - half * (SMALL_T / 2); c < nc; c += SMALL_T) {
-        // the face between positions s and s+1 of line l
-        int l, s;
-        tl.of_slot(c, l, s);
-        int w[S];
+    if constexpr (CHR) {
+        for (int c = threadIdx.x; c < nc; c += SMALL_T) {
+            int l, s, w[S];
+            tl.of_slot(c, l, s);
 #pragma unroll
-        for (int m = 0; m < S; ++m) w[m] = tl.at(s - MID + m) + l * tl.cl;
-#pragma unroll 1
-        for (int q = q0; q < q1; ++q) {
-            const double* fp = F + q * nc;
-            const double* fm = fp + 5 * nc;
-            double a[S], bm[S];
+            for (int m = 0; m < S; ++m) w[m] = tl.at(s - MID + m) + l * tl.cl;
+            double face[5];
+            char_face_fast<DIR, RC>(P, F, g, nc, w, face);
+            if (any_nonfinite(face)) {
+                double wl[5], wr[5], fc[5];
+                int wi[S];
+                const long long il = tl.id(l, s), ir = tl.id(l, s + 1 == tl.len ? 0 : s + 1);
+                wl[0] = W.rho[il]; wl[1] = W.u[il]; wl[2] = W.v[il]; wl[3] = W.w[il]; wl[4] = W.p[il];
+                wr[0] = W.rho[ir]; wr[1] = W.u[ir]; wr[2] = W.v[ir]; wr[3] = W.w[ir]; wr[4] = W.p[ir];
 #pragma unroll
-            for (int m = 0; m < S; ++m) {
-                a[m] = fp[w[m]];
-                bm[S - 1 - m] = fm[w[m]];  // reconstruct_select reverses for flag < 0
+                for (int m = 0; m < S; ++m) wi[m] = w[m];
+                char_face_cold<DIR, RC>(P, wl, wr, F, nc, wi, fc);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) face[q] = fc[q];
             }
-            double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
-                       reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
-            if constexpr (RC == RC_WENO5) {  // as in recon_face
-                if (!finite_hi(f))
-                    f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
-                        weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
-            }
-            fl[q * nc + c] = f;
+#pragma unroll
+            for (int q = 0; q < 5; ++q) fl[q * nc + c] = face[q];
         }
-        if (two) break;
+    } else {
+        // a thread takes a face's components one after the other; of a block with no
+        // more cells than half its threads two threads share them
+        const bool two = nc <= SMALL_T / 2;
+        const int half = two && threadIdx.x >= SMALL_T / 2 ? 1 : 0;
+        const int q0 = half ? 3 : 0, q1 = two && !half ? 3 : 5;
+        for (int c = threadIdx.x - half * (SMALL_T / 2); c < nc; c += SMALL_T) {
+            // the face between positions s and s+1 of line l
+            int l, s;
+            tl.of_slot(c, l, s);
+            int w[S];
+#pragma unroll
+            for (int m = 0; m < S; ++m) w[m] = tl.at(s - MID + m) + l * tl.cl;
+#pragma unroll 1
+            for (int q = q0; q < q1; ++q) {
+                const double* fp = F + q * nc;
+                const double* fm = fp + 5 * nc;
+                double a[S], bm[S];
+#pragma unroll
+                for (int m = 0; m < S; ++m) {
+                    a[m] = fp[w[m]];
+                    bm[S - 1 - m] = fm[w[m]];  // reconstruct_select reverses for flag < 0
+                }
+                double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
+                           reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
+                if constexpr (RC == RC_WENO5) {  // as in recon_face
+                    if (!finite_hi(f))
+                        f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
+                            weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
+                }
+                fl[q * nc + c] = f;
+            }
+            if (two) break;
+        }
     }
     __syncthreads();
     const double inv_h = DIR == 0 ? P.inv_dx : (DIR == 1 ? P.inv_dy : P.inv_dz);
@@ -175,8 +312,8 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
 
 // t3: 15 blocks of n, the x, y and z terms of the five components; fv: the
 // viscous fluxes in store_fv's layout.
-template <int FVS, int RC>
-__global__ void __launch_bounds__(SMALL_T, 512 / SMALL_T)
+template <int FVS, int RC, bool CHR>
+__global__ void __launch_bounds__(SMALL_T, (CHR ? 384 : 512) / SMALL_T)
 k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restrict__ fv, SmallShape sh,
              const Ctrl* __restrict__ ctrl) {
     pdl_enter();
@@ -185,17 +322,17 @@ k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restri
     const long long n = P.n;
     int b = blockIdx.x;
     if (b < sh.nb[0]) {
-        small_sweep<0, FVS, RC>(P, W, t3, b, sh.lb[0], small_sm);
+        small_sweep<0, FVS, RC, CHR>(P, W, t3, b, sh.lb[0], small_sm);
         return;
     }
     b -= sh.nb[0];
     if (b < sh.nb[1]) {
-        small_sweep<1, FVS, RC>(P, W, t3 + 5 * n, b, sh.lb[1], small_sm);
+        small_sweep<1, FVS, RC, CHR>(P, W, t3 + 5 * n, b, sh.lb[1], small_sm);
         return;
     }
     b -= sh.nb[1];
     if (b < sh.nb[2]) {
-        small_sweep<2, FVS, RC>(P, W, t3 + 10 * n, b, sh.lb[2], small_sm);
+        small_sweep<2, FVS, RC, CHR>(P, W, t3 + 10 * n, b, sh.lb[2], small_sm);
         return;
     }
     b -= sh.nb[2];

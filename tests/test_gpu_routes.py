@@ -52,8 +52,14 @@ KW = [dict(), dict(sw_entropy_eps=1e-3, vis_scheme="C6th"), dict(fvs_type="LaxFr
       dict(recon="UD7L", vis_scheme="C4th"), dict(recon="LINEAR"), dict(recon="MDCD_HYBRID")]
 
 
-@pytest.mark.parametrize("kw", KW, ids=scheme_id)
-@pytest.mark.parametrize("box", BOXES, ids=lambda b: "x".join(map(str, b)))
+CHAR_KW = [dict(char_recon="true"), dict(char_recon="true", fvs_type="LaxFriedrichs", recon="MDCD", vis_scheme="C4th"),
+           dict(char_recon="true", recon="UPWIND_7TH"), dict(char_recon="true", recon="MDCD_HYBRID"),
+           dict(char_recon="true", recon="LINEAR")]
+CHAR_BOXES = [(8, 8, 8), (33, 17, 9), (300, 8, 9), (8, 300, 9), (9, 8, 298), (32, 24, 16)]
+
+
+@pytest.mark.parametrize("box,kw", [(b, k) for k in KW for b in BOXES] + [(b, k) for k in CHAR_KW for b in CHAR_BOXES],
+                         ids=lambda v: scheme_id(v) if isinstance(v, dict) else "x".join(map(str, v)))
 def test_small_box_kernel_bits(box, kw):
     p, W = _box_params(box, **kw), _field(box)
     out = []
@@ -190,7 +196,8 @@ EXTREME = [("p", 1e160), ("p", np.inf), ("u", np.nan), ("u", 1e200), ("rho", 1e3
 
 
 @pytest.mark.parametrize("small", ["0", "10000000"], ids=["marching", "small"])
-@pytest.mark.parametrize("kw", [dict(), dict(sw_entropy_eps=1e-3), dict(fvs_type="LaxFriedrichs")], ids=scheme_id)
+@pytest.mark.parametrize("kw", [dict(), dict(sw_entropy_eps=1e-3), dict(fvs_type="LaxFriedrichs"),
+                                dict(char_recon="true")], ids=scheme_id)
 @pytest.mark.parametrize("what", EXTREME, ids=lambda w: f"{w[0]}={w[1]:g}")
 def test_extreme_cell_matches_oracle(oracle_mod, what, kw, small):
     """One extreme cell: the right-hand side is NaN and infinite where the
