@@ -808,20 +808,7 @@ __device__ __forceinline__ R reconstruct(const R* s, const R* lin, R disp, R dis
 // an infinity is NaN either way). DYN: P and M take a loop variable there (a
 // window in shared memory; one in registers needs q at compile time).
 template <class R, int RC, bool DYN, class GP, class GM>
-__device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R diss, R face[5]) {
-    constexpr int S = Stencil<RC>::S;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-        R a[S], b[S];
-#pragma unroll
-        for (int m = 0; m < S; ++m) {
-            a[m] = P(m, q);
-            b[m] = M(m, q);
-        }
-        const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
-        const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
-        face[q] = plus_face + minus_face;
-    }
+__device__ __forceinline__ void recon_face_nonfinite(GP P, GM M, R face[5]) {
     if constexpr (sizeof(R) == 8 && RC == RC_WENO5) {
         if (any_nonfinite(face)) {
 #pragma unroll(DYN ? 1 : 5)
@@ -836,6 +823,62 @@ __device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R d
             }
         }
     }
+}
+
+template <class R, int RC, bool DYN, class GP, class GM>
+__device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R diss, R face[5]) {
+    constexpr int S = Stencil<RC>::S;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        R a[S], b[S];
+#pragma unroll
+        for (int m = 0; m < S; ++m) {
+            a[m] = P(m, q);
+            b[m] = M(m, q);
+        }
+        const R plus_face = reconstruct<R, RC>(a, lin, disp, diss);
+        const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
+        face[q] = plus_face + minus_face;
+    }
+    recon_face_nonfinite<R, RC, DYN>(P, M, face);
+}
+
+// recon_face of the FP64 form from 16-byte words: X(m, k) is word k of window
+// position m, (F+0,F+1) (F+2,F+3) (F-0,F-1) (F-2,F-3) (F+4,F-4), unreversed. Half
+// the shared-memory wavefronts of loading the components one by one, whose
+// 16-byte stride conflicts two ways: 240 a face and warp of a six-point linear
+// scheme, which bound its sweeps (128^3 MDCD).
+template <int RC, class GX>
+__device__ __forceinline__ void recon_words(GX X, const double* lin, double disp, double diss,
+                                            double face[5]) {
+    constexpr int S = Stencil<RC>::S;
+    double a[S], b[S];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        double2 p[S], m2[S];
+#pragma unroll
+        for (int m = 0; m < S; ++m) {
+            p[m] = X(m, k);
+            m2[m] = X(m, 2 + k);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int m = 0; m < S; ++m) {
+                a[m] = h ? p[m].y : p[m].x;
+                b[m] = h ? m2[S - 1 - m].y : m2[S - 1 - m].x;
+            }
+            face[2 * k + h] = reconstruct<double, RC>(a, lin, disp, diss) +
+                              reconstruct<double, RC>(b, lin, disp, diss);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < S; ++m) {
+        const double2 e = X(m, 4);
+        a[m] = e.x;
+        b[S - 1 - m] = e.y;
+    }
+    face[4] = reconstruct<double, RC>(a, lin, disp, diss) + reconstruct<double, RC>(b, lin, disp, diss);
 }
 
 // ---------------------------------------------------------------------------

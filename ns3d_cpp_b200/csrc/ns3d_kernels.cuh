@@ -658,9 +658,14 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
             }
         } else {
             // scalar reconstructions: one component of the window at a time
-            recon_face<R, RC, true>([&](int m, int q) { return ring.comp(wq, cell[m], q, false); },
-                                    [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); },
-                                          lin, disp, diss, face);
+            auto P = [&](int m, int q) { return ring.comp(wq, cell[m], q, false); };
+            auto M = [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); };
+            if constexpr (sizeof(R) == 8) {
+                recon_words<RC>([&](int m, int k) { return ring.a[wq][k][cell[m]]; }, lin, disp, diss, face);
+                recon_face_nonfinite<R, RC, true>(P, M, face);
+            } else {
+                recon_face<R, RC, true>(P, M, lin, disp, diss, face);
+            }
         }
     };
 
@@ -1630,9 +1635,14 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
                 int sl[S];
 #pragma unroll
                 for (int m = 0; m < S; ++m) sl[m] = ph + m < S ? ph + m : ph + m - S;
-                recon_face<R, RC, true>([&](int m, int q) { return ring.comp(sl[m], tid, q, false); },
-                                        [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); },
-                                              lin, disp, diss, face);
+                auto P = [&](int m, int q) { return ring.comp(sl[m], tid, q, false); };
+                auto M = [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); };
+                if constexpr (sizeof(R) == 8) {
+                    recon_words<RC>([&](int m, int k) { return ring.a[sl[m]][k][tid]; }, lin, disp, diss, face);
+                    recon_face_nonfinite<R, RC, true>(P, M, face);
+                } else {
+                    recon_face<R, RC, true>(P, M, lin, disp, diss, face);
+                }
             }
             if (t > 0) {
                 R tz[5];
