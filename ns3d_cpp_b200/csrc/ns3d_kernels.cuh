@@ -51,6 +51,10 @@ enum : int { STOP_NONE = 0, STOP_TOTAL_TIME = 1, STOP_DT_SMALL = 2, STOP_NONPHYS
 
 constexpr double CFL_INIT = 1e9;     // timestep.cpp:8
 
+// Asks for the line of an address in L2, without a register or a wait.
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
 __device__ __forceinline__ int wrap1(int s, int len) {
     return s < 0 ? s + len : (s >= len ? s - len : s);
 }
@@ -430,7 +434,8 @@ k_sweep_x_warp_f32(DevParams P, StateView W, float* __restrict__ tacc, const Ctr
 // __syncwarp per chunk then makes it visible. Chunk 0's double split serves
 // as the row's offset (lane 0's value). Faces, the periodic seam and the
 // T_acc writes as in x_sweep_row.
-template <int FVS, int RC, int ENT>
+// PF: the lines of the loads two chunks on are asked for in L2 (see k_sweep_pipe).
+template <int FVS, int RC, int ENT, bool PF>
 __global__ void __launch_bounds__(32 * XW_WARPS, 4)
 k_sweep_x_pipe(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
     pdl_enter();
@@ -514,6 +519,11 @@ k_sweep_x_pipe(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* _
 #pragma unroll
             for (int q = 0; q < 5; ++q) cr[q] = nxt[q];
             load_raw(min(c + 3, nch - 1), nxt);
+            if (PF && c + 5 < nch) {
+                const long long pid = base + ((c + 5) << 5) + lane;
+                prefetch_l2(W.rho + pid); prefetch_l2(W.u + pid); prefetch_l2(W.v + pid);
+                prefetch_l2(W.w + pid); prefetch_l2(W.p + pid);
+            }
         }
         int cell[S];
 #pragma unroll
@@ -1680,7 +1690,10 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
 #ifndef NS3D_PIPE_MINB
 #define NS3D_PIPE_MINB 3
 #endif
-template <int DIR, int FVS, int RC, int ENT>
+// PF: the lines of the loads two iterations on are asked for in L2 (a linear
+// scheme's iteration is too short to cover a DRAM load: long scoreboard 1.9
+// stalls per issue at 192^3), see prefetched() in the launchers.
+template <int DIR, int FVS, int RC, int ENT, bool PF>
 __global__ void __launch_bounds__(RingCfg<float>::T, NS3D_PIPE_MINB)
 k_sweep_pipe(DevParams P, StateView W, float* __restrict__ tacc, int seg,
              const Ctrl* __restrict__ ctrl) {
@@ -1762,6 +1775,15 @@ k_sweep_pipe(DevParams P, StateView W, float* __restrict__ tacc, int seg,
         for (int q = 0; q < 5; ++q) cur[q] = nxt[q];
         load_raw(f - MID + S + 1, nxt);  // split in the next iteration
         const long long oid = base + (long long)f * stride;
+        if constexpr (PF) {
+            if (f + 2 < c1) {
+                const long long pid = base + (long long)wrap1(f - MID + S + 2, len) * stride;
+                prefetch_l2(W.rho + pid); prefetch_l2(W.u + pid); prefetch_l2(W.v + pid);
+                prefetch_l2(W.w + pid); prefetch_l2(W.p + pid);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) prefetch_l2(tacc + q * n + oid + 2 * stride);
+            }
+        }
         float old[5];
         if (t > 0) {
 #pragma unroll
