@@ -742,6 +742,120 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
     }
 }
 
+// FP32-form x sweep of boxes whose rows are no multiple of 32: k_sweep<0>'s march
+// (one thread per row, its segments, offsets and operations: same bits) with the
+// state and T_acc staged through shared memory. Marching threads of 32 rows
+// touch 32 separate sectors per load and store, which bound that kernel (115 us at
+// 150 x 100 x 130 UD7L against 69 of the y sweep; here 85); here a block of 128 rows copies eight
+// columns at a time, eight consecutive lanes to a row, and takes its rows across
+// the j and k limits, so that only the last block has idle threads.
+constexpr int XR_T = 128, XR_C = 8, XR_P = XR_T + 1;  // rows, columns, padded rows
+constexpr size_t XR_SMEM = (size_t)5 * XR_C * XR_P * (sizeof(double) + sizeof(float));
+
+template <int FVS, int RC>
+__global__ void __launch_bounds__(XR_T, 3)
+k_sweep_x_rows(DevParams P, StateView W, float* __restrict__ tacc, int seg, const Ctrl* __restrict__ ctrl) {
+    pdl_enter();
+    if (ctrl && ctrl->stop) return;
+    constexpr int S = Stencil<RC>::S;
+    constexpr int MID = (S - 1) / 2;
+    extern __shared__ double xr_sm[];
+    double* in = xr_sm;                                               // [5][XR_C][XR_P]
+    float* out = reinterpret_cast<float*>(xr_sm + 5 * XR_C * XR_P);   // [5][XR_C][XR_P]
+    const int nx = P.nx, tid = threadIdx.x;
+    const long long n = P.n, r0 = (long long)blockIdx.x * XR_T;
+    const int nr = (int)min((long long)XR_T, (long long)P.ny * P.nz - r0);
+    const int c0 = blockIdx.y * seg, c1 = min(c0 + seg, nx);
+    // the march's cells: s0 + i, i = 0 .. total-1; cell i completes the window of
+    // a face from i = S-1 on and the difference of cell c0 + i - S from i = S on
+    const int s0 = c0 - 1 - MID, total = c1 - c0 + S;
+    float lin[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) lin[m] = float(P.lin[m]);
+    const float disp = float(P.mdcd_disp), diss = float(P.mdcd_diss);
+    const float inv_h = float(P.inv_dx);
+    const double inv_gm1 = 1.0 / (P.gamma - 1.0), inv_2g = 1.0 / (2.0 * P.gamma);
+    const double* src[5] = {W.rho, W.u, W.v, W.w, W.p};
+    const int lx = tid % XR_C, lr = tid / XR_C;
+    auto flush = [&](int i0) {  // the chunk of cells i0 .. i0+XR_C-1
+        const int i = i0 + lx;
+        if (i < S || i >= total) return;
+        for (int r = lr; r < nr; r += XR_T / XR_C)
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+                tacc[q * n + (r0 + r) * nx + c0 + i - S] = out[(q * XR_C + lx) * XR_P + r];
+    };
+    float fp[S][5], fm[S][5], prev[5];
+    double refp[5], refm[5];
+    // k_sweep's split_raw: the first cell sets the offset
+    auto split_raw = [&](const double* raw, float* Fp, float* Fm, bool set_ref) {
+        double Fpd[5], Fmd[5];
+        split_fast<FVS, 1, 0, 0>(P, inv_gm1, inv_2g, raw, Fpd, Fmd);
+        if (set_ref) {
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                refp[q] = Fpd[q];
+                refm[q] = Fmd[q];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            Fp[q] = float(Fpd[q] - refp[q]);
+            Fm[q] = float(Fmd[q] - refm[q]);
+        }
+    };
+    int i = 0;
+    for (int i0 = 0; i0 < total; i0 += XR_C) {
+        if (i0 > 0) flush(i0 - XR_C);
+        if (i0 + lx < total) {
+            const int s = wrap1(s0 + i0 + lx, nx);
+#pragma unroll
+            for (int k = 0; k < XR_C; ++k) {
+                const int r = lr + k * (XR_T / XR_C);
+                if (r < nr) {
+#pragma unroll
+                    for (int v = 0; v < 5; ++v) in[(v * XR_C + lx) * XR_P + r] = src[v][(r0 + r) * nx + s];
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < nr) {
+#pragma unroll 1
+            for (int x = 0; x < XR_C && i < total; ++x, ++i) {
+                double raw[5];
+#pragma unroll
+                for (int v = 0; v < 5; ++v) raw[v] = in[(v * XR_C + x) * XR_P + tid];
+                // the window moves on by one cell
+#pragma unroll
+                for (int m = 0; m < S - 1; ++m)
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        fp[m][q] = fp[m + 1][q];
+                        fm[m][q] = fm[m + 1][q];
+                    }
+                if (i == 0) split_raw(raw, fp[S - 1], fm[S - 1], true);
+                else split_raw(raw, fp[S - 1], fm[S - 1], false);
+                if (i < S - 1) continue;
+                float face[5];
+                if constexpr (RC == RC_WENO5) {
+                    weno5_face_x2([&](int m, int q) { return fp[m][q]; },
+                                  [&](int m, int q) { return fm[S - 1 - m][q]; }, face);
+                } else {
+                    recon_face<float, RC, false>([&](int m, int q) { return fp[m][q]; },
+                                                 [&](int m, int q) { return fm[S - 1 - m][q]; }, lin, disp, diss, face);
+                }
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+                    if (i >= S) out[(q * XR_C + x) * XR_P + tid] = (face[q] - prev[q]) * inv_h;
+                    prev[q] = face[q];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    flush((total - 1) / XR_C * XR_C);
+}
+
 // ---------------------------------------------------------------------------
 // Viscous flux storage (fv). FP64 form: 9 blocks of n in the order 0 xx, 1 yy,
 // 2 zz, 3 xy, 4 xz, 5 yz, 6 ex, 7 ey, 8 ez. FP32 form: three float4 blocks of

@@ -166,6 +166,23 @@ cudaError_t by_split(const DevParams& P, F f) {
     return by_pf(std::integral_constant<int, 0>{});
 }
 
+// k_sweep_x_rows: 62 KB of dynamic shared memory, opted in once per
+// instantiation and device.
+template <int FVS, int RC>
+cudaError_t x_rows(const LaunchCfg& L, StateView W, float* tacc, int seg, const Ctrl* ctrl) {
+    static bool opted[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !opted[dev]) {
+        e = cudaFuncSetAttribute(k_sweep_x_rows<FVS, RC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XR_SMEM);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) opted[dev] = true;
+    }
+    const dim3 grid((unsigned)(((long long)L.P.ny * L.P.nz + XR_T - 1) / XR_T), (L.P.nx + seg - 1) / seg);
+    return launch_pdl(L, k_sweep_x_rows<FVS, RC>, grid, XR_T, XR_SMEM, L.P, W, tacc, seg, ctrl);
+}
+
 template <int DIR, class R, int FVS, int RC, bool CHR>
 cudaError_t sweep_dir(const LaunchCfg& L, StateView W, R* tacc, const Ctrl* ctrl) {
     const DevParams& P = L.P;
@@ -198,6 +215,13 @@ cudaError_t sweep_dir(const LaunchCfg& L, StateView W, R* tacc, const Ctrl* ctrl
             P, W, tacc, m.seg, ctrl, FuseArgs<R>{});
     } else {
         const MarchShape m = march_shape<DIR>(L, 128);
+        // Lax-Friedrichs only: beside another loop the compiler contracts the
+        // Steger-Warming split's sums into other FMAs, and the float deviations'
+        // roundings flip. Below 140000 cells a launch has too few blocks (24^3
+        // 76 -> 81 us a step, 40^3 UD7L 211 -> 218; 52x61x47 MDCD 214 -> 184).
+        if constexpr (sizeof(R) == 4 && !CHR && FVS == FV_LF) {
+            if (P.n > 140000) return x_rows<FVS, RC>(L, W, tacc, m.seg, ctrl);
+        }
         return launch_pdl(L, k_sweep<DIR, R, FVS, RC, CHR>, m.grid, m.th, 0, P, W, tacc, m.seg, ctrl);
     }
 }

@@ -13,7 +13,7 @@ import pytest
 
 import ns3d_cpp_b200 as ns
 from ns3d_cpp_b200 import initial
-from conftest import ref_cfg, scheme_id
+from conftest import ref_cfg, relerr, scheme_id
 from test_gpu_parity import params_from_cfg
 
 pytestmark = pytest.mark.gpu
@@ -73,6 +73,26 @@ def test_small_box_kernel_bits(box, kw):
     assert np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2]
     assert out[1][3] > out[0][3]  # the second context took the kernel (its terms are kept apart)
+
+
+# k_sweep_x_rows (FP32 form, Lax-Friedrichs, nx no multiple of 32, more than
+# 140000 cells): one segment and several, a last block of rows that is not
+# full, columns that are no multiple of eight, against the oracle with the FP32
+# form's bound on the right-hand side (5e-5 of each variable's largest value)
+@pytest.mark.parametrize("kw", [dict(), dict(recon="MDCD"), dict(recon="UD7L"), dict(recon="LINEAR")], ids=scheme_id)
+@pytest.mark.parametrize("box", [(70, 51, 41), (9, 130, 121), (500, 17, 18)], ids=lambda b: "x".join(map(str, b)))
+def test_fp32_x_rows_matches_oracle(oracle_mod, box, kw):
+    cfg = ref_cfg(16, Ma=0.3, Re=400, fvs_type="LaxFriedrichs", **kw)
+    cfg.update(global_nx=box[0], global_ny=box[1], global_nz=box[2])
+    nx, ny, nz = box
+    Z, Y, X = np.meshgrid(*[np.arange(m) * (2 * np.pi / m) for m in (nz, ny, nx)], indexing="ij")
+    W = np.stack([1 + 0.1 * np.sin(X + 0.3) * np.cos(Y + Z), np.sin(X) * np.cos(Y) * np.cos(Z),
+                  -np.cos(X) * np.sin(Y) * np.cos(Z) + 0.1, 0.3 * np.sin(Z + X),
+                  7.9 + 0.5 * np.cos(2 * X) * np.cos(Y + Z)])
+    with ns.Solver(params_from_cfg(cfg).replace(precision="fp32acc64")) as s:
+        s.upload_primitive(W)
+        got = s.compute_rhs()
+    assert np.all(relerr(got, oracle_mod.Oracle(cfg).rhs(W)) <= 5e-5)
 
 
 def test_small_box_stop_leaves_state():
