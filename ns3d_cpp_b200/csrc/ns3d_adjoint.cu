@@ -428,6 +428,7 @@ template <int FVS, int RC>
 __global__ void __launch_bounds__(ADJ_T, 4)
 k_adj_flux(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ gw,
            double* __restrict__ lg, SmallShape sh) {
+    pdl_enter();
     extern __shared__ double adj_sm[];
     const long long n = P.n;
     int b = blockIdx.x;
@@ -497,6 +498,7 @@ __global__ void __launch_bounds__(128)
 k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const double* __restrict__ lg,
              double* lamW, int finish, int next, StateView Wp, double* __restrict__ lamU0,
              double* __restrict__ lamR, double dt) {
+    pdl_enter();
     const long long n = P.n;
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
@@ -575,9 +577,8 @@ cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double
         // 128 to 256 cells a block: several blocks per SM, at least two per SM for each direction
         const long long target = std::min(256ll, std::max(64ll, 3 * P.n / (2 * 148)));
         const SmallShape sh = small_shape(P, target, ADJ_NC, ADJ_T);
-        k_adj_flux<FVS, RC><<<small_blocks(sh), ADJ_T, adj_smem<RC>(small_cells(P, sh)), L.stream>>>(P, W, lamR, gw,
-                                                                                                   lg, sh);
-        return cudaGetLastError();
+        return launch_pdl(L, k_adj_flux<FVS, RC>, small_blocks(sh), ADJ_T, adj_smem<RC>(small_cells(P, sh)), P, W,
+                          lamR, gw, lg, sh);
     }
     cudaError_t e = adj_dir<0, FVS, RC>(L, W, lamR, G, gw);
     if (e == cudaSuccess) e = adj_dir<1, FVS, RC>(L, W, lamR, G, gw);
@@ -621,12 +622,12 @@ cudaError_t adj_rhs_vjp(const LaunchCfg& L, StateView W, double* G, double* lg, 
                                    : adj_flux_rc<FV_LF>(L, W, lamR, Gw, gw, lg);
     if (e != cudaSuccess) return e;
     const unsigned b = (unsigned)((P.n + 127) / 128);
-    switch (P.vis_order) {
-    case 4: k_adj_reduce<4><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
-    case 6: k_adj_reduce<6><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
-    default: k_adj_reduce<8><<<b, 128, 0, L.stream>>>(P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt); break;
-    }
-    return cudaGetLastError();
+    auto reduce = [&](auto kernel) {
+        return launch_pdl(L, kernel, b, 128, 0, P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt);
+    };
+    if (P.vis_order == 4) return reduce(k_adj_reduce<4>);
+    if (P.vis_order == 6) return reduce(k_adj_reduce<6>);
+    return reduce(k_adj_reduce<8>);
 }
 
 cudaError_t adj_stage(const LaunchCfg& L, int stage, StateView Wk, StateView Wp, const double* lamWk, double* lamU0,
