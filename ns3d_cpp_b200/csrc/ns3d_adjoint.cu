@@ -428,7 +428,7 @@ template <int FVS, int RC>
 __global__ void __launch_bounds__(ADJ_T, 4)
 k_adj_flux(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ gw,
            double* __restrict__ lg, SmallShape sh) {
-    pdl_enter();
+    pdl_enter(P);
     extern __shared__ double adj_sm[];
     const long long n = P.n;
     int b = blockIdx.x;
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(128)
 k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const double* __restrict__ lg,
              double* lamW, int finish, int next, StateView Wp, double* __restrict__ lamU0,
              double* __restrict__ lamR, double dt) {
-    pdl_enter();
+    pdl_enter(P);
     const long long n = P.n;
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;

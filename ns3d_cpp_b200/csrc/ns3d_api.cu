@@ -756,8 +756,8 @@ void default_tiling(LaunchCfg& L) {
     L.pipe = 3;   // FP32 sweeps with the software-pipelined split (k_sweep_x_pipe, k_sweep_pipe)
     // an override of the marching kernels' shapes selects those kernels
     L.small = 1500000;
-    L.pdl = 1;  // where pdl_box() holds
-    if (const char* e = std::getenv("NS3D_PDL")) L.pdl = std::atoi(e);
+    L.P.pdl = 1;  // where pdl_box() holds
+    if (const char* e = std::getenv("NS3D_PDL")) L.P.pdl = std::atoi(e);
     for (const char* v : {"NS3D_TILE_ZB", "NS3D_TILED", "NS3D_SEG"})
         if (std::getenv(v)) L.small = 0;
     if (const char* e = std::getenv("NS3D_SMALL")) L.small = std::atoll(e);
@@ -845,7 +845,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     ctx->L.chr = q.char_recon ? 1 : 0;
     for (int d = 0; d < 3; ++d) ctx->L.seg[d] = 0;  // chosen per launch from the grid
     default_tiling(ctx->L);
-    if (!pdl_box(ctx->L, q.precision == NS3D_PREC_FP64)) ctx->L.pdl = 0;
+    if (!pdl_box(ctx->L, q.precision == NS3D_PREC_FP64)) ctx->L.P.pdl = 0;
     ctx->rsize = q.precision == NS3D_PREC_FP64 ? sizeof(double) : sizeof(float);
 
     auto bail = [&](ns3d_status st, const std::string& m) {
@@ -860,7 +860,7 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     ctx->L.stream = ctx->stream;
     if (const char* ov = std::getenv("NS3D_OVERLAP")) ctx->overlap = std::atoi(ov) != 0;
     if (const char* fu = std::getenv("NS3D_FUSE")) ctx->fuse = std::atoi(fu) != 0;
-    if (ctx->overlap) ctx->L.pdl = 0;  // kernels of two streams depend on each other
+    if (ctx->overlap) ctx->L.P.pdl = 0;  // kernels of two streams depend on each other
     if (ctx->overlap &&
         (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
          cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||

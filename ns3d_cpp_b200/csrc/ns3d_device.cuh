@@ -38,6 +38,7 @@ struct DevParams {
     double lin[8];   // linear reconstruction coefficients (LIN6 / LIN8)
     double mdcd_disp, mdcd_diss;
     int vis_order;   // 4, 6, 8
+    int pdl;         // 1: the launches overlap (launch_pdl, pdl_enter)
     // divisors of the central derivatives (12 h, 60 h or h) along x, y, z, and
     // the reciprocals RN(1/b) of these, of the heat flux's Pr and of the
     // split's 2 gamma (see quot_rcp)

@@ -66,9 +66,15 @@ __device__ __forceinline__ int wrap1(int s, int len) {
 // attribute waits before its first read or write of device memory.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() {
-    pdl_wait();
-    pdl_trigger();
+// At a kernel's entry. In boxes whose launches do not overlap (P.pdl 0) neither
+// instruction is executed: they cost every block up to a microsecond, which
+// narrow boxes, whose launches have tens of thousands of blocks of a few live threads,
+// felt in full (FP32 10 x 500 x 100: k_update 62.6 us without them, 72.1 with).
+__device__ __forceinline__ void pdl_enter(const DevParams& P) {
+    if (P.pdl) {
+        pdl_wait();
+        pdl_trigger();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -228,7 +234,7 @@ __device__ __forceinline__ void ring_window_at(int ph, const SplitRing<R, S, T>&
 template <int DIR, class R, int FVS, int RC, bool CHR = false>
 __global__ void __launch_bounds__(128)
 k_sweep(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
@@ -399,7 +405,7 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
 template <class R, int FVS, int RC, bool CHR = false>
 __global__ void __launch_bounds__(32 * XW_WARPS)
 k_sweep_x_warp(DevParams P, StateView W, R* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     __shared__ SplitRing<R, XW_WARPS, 96> ring;  // [warp][3 chunks x 32 cells]
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
@@ -415,7 +421,7 @@ k_sweep_x_warp(DevParams P, StateView W, R* __restrict__ tacc, const Ctrl* __res
 template <int FVS, int RC>
 __global__ void __maxnreg__(128)
 k_sweep_x_warp_f32(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     __shared__ SplitRing<float, XW_WARPS, 96> ring;
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
@@ -438,7 +444,7 @@ k_sweep_x_warp_f32(DevParams P, StateView W, float* __restrict__ tacc, const Ctr
 template <int FVS, int RC, int ENT, bool PF>
 __global__ void __launch_bounds__(32 * XW_WARPS, 4)
 k_sweep_x_pipe(DevParams P, StateView W, float* __restrict__ tacc, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
@@ -755,7 +761,7 @@ constexpr size_t XR_SMEM = (size_t)5 * XR_C * XR_P * (sizeof(double) + sizeof(fl
 template <int FVS, int RC>
 __global__ void __launch_bounds__(XR_T, 3)
 k_sweep_x_rows(DevParams P, StateView W, float* __restrict__ tacc, int seg, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
@@ -968,7 +974,7 @@ __device__ __forceinline__ void visc_cell(const DevParams& P, const StateView& W
 template <class R, int ORD>
 __global__ void __launch_bounds__(128)
 k_visc_flux(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.nx) return;
@@ -999,7 +1005,7 @@ k_visc_flux_25d(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __rest
                 int zb) {
     constexpr int VT_X = VTile<R>::X, VT_Y = VTile<R>::Y, VT_H = VTile<R>::H;
     constexpr int VT_SX = VTile<R>::SX, VT_SY = VTile<R>::SY;
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     // FP32-stencil form: values enter the tile and the z queue as float
     // deviations from one reference per block and variable (formed in
@@ -1147,7 +1153,7 @@ k_visc_flux_pipe(DevParams P, StateView W, R* __restrict__ fv, const Ctrl* __res
     using VP = VPipe<R>;
     constexpr int X = VT::X, Y = VT::Y, H = VT::H, SX = VT::SX, SY = VT::SY;
     constexpr int NT = VP::NT, NH = VP::NH, HPT = VP::HPT;
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     constexpr bool kDeviation = sizeof(R) < sizeof(double);
     extern __shared__ __align__(16) unsigned char vsm[];
@@ -1585,7 +1591,7 @@ template <class R, int ORD, int STAGE, bool T3 = false>
 __global__ void __launch_bounds__(128, 8)
 k_update(DevParams P, StateView Wc, StateView W0, const R* __restrict__ tacc,
          const R* __restrict__ fv, StateOut Wn, Ctrl* ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl->stop) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < P.nx;
@@ -1661,7 +1667,7 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
     constexpr int T = RingCfg<R>::T;
     constexpr bool kDeviation = sizeof(R) < sizeof(double);
     __shared__ SplitRing<R, S, T> ring;
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long n = P.n;
@@ -1816,7 +1822,7 @@ k_sweep_pipe(DevParams P, StateView W, float* __restrict__ tacc, int seg,
     constexpr int MID = (S - 1) / 2;
     constexpr int T = RingCfg<float>::T;
     __shared__ SplitRing<float, S, T> ring;
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     const int nx = P.nx, ny = P.ny, nz = P.nz;
     const long long n = P.n;
@@ -2028,7 +2034,8 @@ __device__ void control_post(Ctrl* c, int mode, double total_time, long long n, 
 enum : int { CONTROL_POST = 1, CONTROL_PRE = 2 };
 __global__ void k_control(Ctrl* c, int what, int mode, double cfl, double dt_fixed, double total_time,
                           double out_freq, long long n, double* times) {
-    pdl_enter();
+    pdl_wait();
+    pdl_trigger();
     if (what & CONTROL_POST) control_post(c, mode, total_time, n, times);
     if (what & CONTROL_PRE) control_pre(c, mode, cfl, dt_fixed, total_time, out_freq);
 }

@@ -23,13 +23,12 @@ struct LaunchCfg {
     int zb;       // planes per block of the 2.5-D viscous kernels (0: from the grid)
     int tiled;    // bit 0: 2.5-D visc_flux (when the box tiles); bit 1: its pipelined form
     long long small;  // FP64 boxes of at most so many cells take k_flux_small (see small_box)
-    int pdl;      // 1: programmatic dependent launches (launch_pdl)
     int pipe;     // FP32 sweeps with the software-pipelined split: bit 0 the x sweep
                   // (k_sweep_x_pipe, rows of >= 128 cells), bit 1 the y / z sweeps (k_sweep_pipe)
 };
 
-// Launch-shape defaults, overridable by NS3D_TILE_ZB / NS3D_TILED / NS3D_SEG / NS3D_PIPE for
-// tuning.
+// Launch-shape defaults, overridable by NS3D_TILE_ZB / NS3D_TILED / NS3D_SEG / NS3D_PIPE /
+// NS3D_SMALL / NS3D_PDL for tuning.
 void default_tiling(LaunchCfg& L);
 
 // One inviscid sweep (dir 0, 1, 2 in this order per RHS evaluation).
@@ -51,7 +50,7 @@ constexpr long long kSmallUpdateCells = 33000;  // stages of larger boxes: k_upd
 cudaError_t launch_update_small(const LaunchCfg& L, int stage, StateView Wc, StateView W0, const double* tacc,
                                 const double* fv, StateOut Wn, Ctrl* ctrl, double* rhs);
 
-// A launch whose kernel calls pdl_wait: with L.pdl it may start while its
+// A launch whose kernel calls pdl_wait: with P.pdl it may start while its
 // predecessor in the stream drains.
 template <class... K, class... A>
 cudaError_t launch_pdl(const LaunchCfg& L, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, A... args) {
@@ -64,7 +63,7 @@ cudaError_t launch_pdl(const LaunchCfg& L, void (*kernel)(K...), dim3 grid, dim3
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = L.pdl ? 1 : 0;
+    cfg.numAttrs = L.P.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
 }
 // The z sweep fused with the stage update (k_sweep_ring<2, ..., FUSE>): T_acc
@@ -111,13 +110,26 @@ inline bool small_box(const LaunchCfg& L) {
 // 281 -> 266 us; FP32 8^3 101 -> 76 us, 64^3 243 -> 212 us, 96^3 616 -> 587 us). On
 // larger ones the next kernel's waiting blocks cost more than the overlap gains
 // (FP64 128^3 MDCD 1308 -> 1449 us, FP32 90x100x84 651 -> 665), in the FP32
-// form's eight-point schemes earlier (75^3 455 -> 520 us, 64^3 228 -> 197).
+// form's eight-point schemes earlier (75^3 455 -> 520 us, 64^3 228 -> 197). Two
+// shapes of FP32 boxes inside those limits lose, both with launches of many
+// 32-thread blocks whose lanes are not all live, each of which waits and signals:
+// narrow ones with very many rows (10x500x100 C4th linear 570 -> 626 us, LF WENO5
+// 1050 -> 1102; 9x130x121, 15730 rows, gains: 547 -> 519), and of the boxes with nx
+// below 64 and no multiple of 32 those of 55000 to 140000 cells, with the C8th
+// viscous terms or Lax-Friedrichs + WENO5 and all but the two-point scheme (LF MDCD
+// 54x43x47 185 -> 209, 53x26x54 166 -> 183, 49x37x46 180 -> 192, LF WENO5 55x54x46 213 -> 238;
+// smaller and larger ones gain, LF MDCD 34^3 153 -> 141, 52^3 207 -> 183).
 inline bool pdl_box(const LaunchCfg& L, bool fp64) {
-    const long long n = L.P.n;
+    const DevParams& P = L.P;
+    const long long n = P.n;
     if (n <= 30000) return true;
     if (L.chr || L.rc == RC_MDCD_HYBRID) return false;
     if (fp64) return n <= 300000;
-    return n <= 700000 && (L.rc != RC_LIN8 || (L.P.nx % 32 == 0 && n <= 300000));
+    if ((long long)P.ny * P.nz > 30000) return false;
+    if (P.nx < 64 && P.nx % 32 != 0 && n >= 55000 && n <= 140000 && L.rc != RC_LINEAR &&
+        (P.vis_order == 8 || (L.rc == RC_WENO5 && L.fvs == FV_LF)))
+        return false;
+    return n <= 700000 && (L.rc != RC_LIN8 || (P.nx % 32 == 0 && n <= 300000));
 }
 
 #ifdef NS3D_LAUNCH_IMPL

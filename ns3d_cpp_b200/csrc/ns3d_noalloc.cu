@@ -134,7 +134,7 @@ extern "C" ns3d_status ns3d_compute_rhs_noalloc(const ns3d_params* p, const doub
     double* scratch = nullptr;
     if ((s = scratch_address(&scratch)) != NS3D_OK) return s;
     L.stream = static_cast<cudaStream_t>(stream);
-    if (!pdl_box(L, p->precision == NS3D_PREC_FP64)) L.pdl = 0;
+    if (!pdl_box(L, p->precision == NS3D_PREC_FP64)) L.P.pdl = 0;
     double* T = scratch;
     const long long n = L.P.n;
     k_noalloc_temperature<<<(unsigned)((n + 255) / 256), 256, 0, L.stream>>>(n, rho, pres, L.P.Rgas, T);

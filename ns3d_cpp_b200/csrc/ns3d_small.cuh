@@ -316,7 +316,7 @@ template <int FVS, int RC, bool CHR>
 __global__ void __launch_bounds__(SMALL_T, (CHR ? 384 : 512) / SMALL_T)
 k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restrict__ fv, SmallShape sh,
              const Ctrl* __restrict__ ctrl) {
-    pdl_enter();
+    pdl_enter(P);
     if (ctrl && ctrl->stop) return;
     extern __shared__ double small_sm[];
     const long long n = P.n;
@@ -356,10 +356,11 @@ template <int ORD, int STAGE>
 __global__ void __launch_bounds__(160)
 k_update_small(DevParams P, StateView Wc, StateView W0, const double* __restrict__ t3,
                const double* __restrict__ fv, StateOut Wn, Ctrl* ctrl, double* __restrict__ rhs) {
-    pdl_wait();
     if constexpr (STAGE > 0) {
-        pdl_trigger();
+        pdl_enter(P);
         if (ctrl->stop) return;
+    } else {
+        if (P.pdl) pdl_wait();
     }
     __shared__ double rs[5][32];
     const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;

@@ -1,0 +1,54 @@
+"""Launches that must not change a bit when they are overlapped by programmatic
+dependent launch (NS3D_PDL=0, read when a context is created, serialises them)."""
+import numpy as np
+import pytest
+
+from conftest import scheme_id
+from test_gpu_routes import _box_params, _field, _solver
+
+pytestmark = pytest.mark.gpu
+
+
+# boxes of every rule under which launches overlap: FP64 through k_flux_small
+# (component- and characteristic-wise) and through the marching kernels, FP32
+# below and above 30000 cells, eight-point schemes on warp rows
+@pytest.mark.parametrize("precision,box,kw,env", [
+    ("fp64", (16, 12, 10), dict(sw_entropy_eps=1e-3), {}),
+    ("fp64", (64, 24, 31), dict(fvs_type="LaxFriedrichs", recon="MDCD"), {}),
+    ("fp64", (33, 17, 9), dict(char_recon="true"), {}),
+    ("fp64", (20, 18, 16), dict(), {"NS3D_SMALL": "0"}),
+    ("fp64", (64, 48, 32), dict(recon="UD7L", vis_scheme="C4th"), {"NS3D_SMALL": "0"}),
+    ("fp64", (410, 8, 9), dict(), {}),
+    ("fp32acc64", (8, 8, 8), dict(), {}),
+    ("fp32acc64", (24, 20, 16), dict(fvs_type="LaxFriedrichs", recon="MDCD_HYBRID"), {}),
+    ("fp32acc64", (70, 40, 30), dict(sw_entropy_eps=1e-3, vis_scheme="C6th"), {}),
+    ("fp32acc64", (32, 200, 16), dict(recon="LINEAR"), {}),
+    ("fp32acc64", (128, 32, 40), dict(recon="UPWIND_7TH"), {}),
+    ("fp32acc64", (100, 75, 70), dict(fvs_type="LaxFriedrichs"), {}),
+], ids=lambda v: scheme_id(v) if isinstance(v, dict) else ("x".join(map(str, v)) if isinstance(v, tuple) else v))
+def test_overlapped_launches_bits(precision, box, kw, env):
+    p, W, out = _box_params(box, **kw).replace(precision=precision), _field(box), []
+    for pdl in ("0", "1"):
+        with _solver(p, {"NS3D_PDL": pdl, **env}) as s:
+            s.upload_primitive(W)
+            rhs = s.compute_rhs()
+            s.step(12)
+            a = s.download_primitive()
+            s.upload_primitive(W)
+            s.step(5)
+            out.append((rhs, a, s.download_primitive(), s.last_dt()))
+    for q in range(3):
+        assert np.array_equal(out[0][q], out[1][q])
+    assert out[0][3] == out[1][3]
+
+
+@pytest.mark.parametrize("box", [(16, 12, 10), (9, 8, 301)], ids=["flux_kernel", "long_lines"])
+def test_overlapped_adjoint_bits(box):
+    p, W, out = _box_params(box, sw_entropy_eps=1e-3), _field(box), []
+    for pdl in ("0", "1"):
+        with _solver(p, {"NS3D_PDL": pdl}) as s:
+            s.upload_primitive(W)
+            g, J, dts = s.adjoint(5, 2)
+            out.append((g, J, dts, s.rhs_vjp(W), s.download_primitive()))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
