@@ -761,6 +761,8 @@ void default_tiling(LaunchCfg& L) {
     for (const char* v : {"NS3D_TILE_ZB", "NS3D_TILED", "NS3D_SEG"})
         if (std::getenv(v)) L.small = 0;
     if (const char* e = std::getenv("NS3D_SMALL")) L.small = std::atoll(e);
+    L.rows = -1;
+    if (const char* e = std::getenv("NS3D_XROWS")) L.rows = std::atoi(e);
     if (const char* e = std::getenv("NS3D_PIPE")) L.pipe = std::atoi(e);
     if (const char* e = std::getenv("NS3D_TILE_ZB")) L.zb = std::atoi(e);
     if (const char* e = std::getenv("NS3D_TILED")) L.tiled = std::atoi(e);

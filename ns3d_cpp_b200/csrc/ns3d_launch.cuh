@@ -23,12 +23,13 @@ struct LaunchCfg {
     int zb;       // planes per block of the 2.5-D viscous kernels (0: from the grid)
     int tiled;    // bit 0: 2.5-D visc_flux (when the box tiles); bit 1: its pipelined form
     long long small;  // FP64 boxes of at most so many cells take k_flux_small (see small_box)
+    int rows;     // FP32 Lax-Friedrichs x sweep off the warp rows by k_sweep_x_rows: 1 always, 0 never, -1 where x_rows_box() holds
     int pipe;     // FP32 sweeps with the software-pipelined split: bit 0 the x sweep
                   // (k_sweep_x_pipe, rows of >= 128 cells), bit 1 the y / z sweeps (k_sweep_pipe)
 };
 
 // Launch-shape defaults, overridable by NS3D_TILE_ZB / NS3D_TILED / NS3D_SEG / NS3D_PIPE /
-// NS3D_SMALL / NS3D_PDL for tuning.
+// NS3D_SMALL / NS3D_PDL / NS3D_XROWS for tuning.
 void default_tiling(LaunchCfg& L);
 
 // One inviscid sweep (dir 0, 1, 2 in this order per RHS evaluation).
@@ -178,6 +179,25 @@ cudaError_t by_split(const DevParams& P, F f) {
     return by_pf(std::integral_constant<int, 0>{});
 }
 
+// Whether the FP32 Lax-Friedrichs x sweep off the warp rows takes k_sweep_x_rows: it
+// copies eight columns of 128 rows at a time, so it needs cells enough for the
+// grid (24^3 76 -> 81 us a step), more than a chunk or two of columns (10x500x100
+// WENO5 1103 -> 1120 us, 17x90x100 equal, 20x155x154 UD7L 627 -> 581) and segments
+// of several of them (rows/1024 cells each): with 5600 rows every scheme gains
+// (75^3 WENO5 390 -> 373, UD7L 379 -> 366; 100x75x90 509 -> 467, 471 -> 436), with fewer
+// the eight-point window's extra splits lose (70x51x41, 2091 rows, 216 -> 231,
+// 130x40x40 273 -> 304; 4200 rows even) and long rows in WENO5 (501x60x60 1171 -> 1243,
+// 250x60x70 666 -> 679; but 58x44x58 240 -> 200, 60^3 265 -> 249), and with 400 to 1800 rows
+// the rest too (2001x20x20 MDCD 592 -> 672; 70x51x41 167 -> 164, 75x60x50 215 -> 204).
+inline bool x_rows_box(const LaunchCfg& L) {
+    if (L.rows >= 0) return L.rows != 0;
+    const DevParams& P = L.P;
+    const long long rows = (long long)P.ny * P.nz;
+    if (P.n <= 140000 || P.nx < 16) return false;
+    if (rows > 5000) return true;
+    return rows > 2000 && L.rc != RC_LIN8 && (L.rc != RC_WENO5 || P.nx <= 100);
+}
+
 // k_sweep_x_rows: 62 KB of dynamic shared memory, opted in once per
 // instantiation and device.
 template <int FVS, int RC>
@@ -229,10 +249,9 @@ cudaError_t sweep_dir(const LaunchCfg& L, StateView W, R* tacc, const Ctrl* ctrl
         const MarchShape m = march_shape<DIR>(L, 128);
         // Lax-Friedrichs only: beside another loop the compiler contracts the
         // Steger-Warming split's sums into other FMAs, and the float deviations'
-        // roundings flip. Below 140000 cells a launch has too few blocks (24^3
-        // 76 -> 81 us a step, 40^3 UD7L 211 -> 218; 52x61x47 MDCD 214 -> 184).
+        // roundings flip.
         if constexpr (sizeof(R) == 4 && !CHR && FVS == FV_LF) {
-            if (P.n > 140000) return x_rows<FVS, RC>(L, W, tacc, m.seg, ctrl);
+            if (x_rows_box(L)) return x_rows<FVS, RC>(L, W, tacc, m.seg, ctrl);
         }
         return launch_pdl(L, k_sweep<DIR, R, FVS, RC, CHR>, m.grid, m.th, 0, P, W, tacc, m.seg, ctrl);
     }

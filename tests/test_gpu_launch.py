@@ -1,5 +1,7 @@
-"""Launches that must not change a bit when they are overlapped by programmatic
-dependent launch (NS3D_PDL=0, read when a context is created, serialises them)."""
+"""Launch routes that must not change a bit: launches overlapped by programmatic
+dependent launch (NS3D_PDL=0 serialises them), and the FP32 form's staged x
+sweep k_sweep_x_rows (NS3D_XROWS=1 always, 0 never). Both are read when a
+context is created."""
 import numpy as np
 import pytest
 
@@ -24,7 +26,7 @@ pytestmark = pytest.mark.gpu
     ("fp32acc64", (70, 40, 30), dict(sw_entropy_eps=1e-3, vis_scheme="C6th"), {}),
     ("fp32acc64", (32, 200, 16), dict(recon="LINEAR"), {}),
     ("fp32acc64", (128, 32, 40), dict(recon="UPWIND_7TH"), {}),
-    ("fp32acc64", (100, 75, 70), dict(fvs_type="LaxFriedrichs"), {}),
+    ("fp32acc64", (100, 75, 70), dict(fvs_type="LaxFriedrichs"), {"NS3D_XROWS": "1"}),
 ], ids=lambda v: scheme_id(v) if isinstance(v, dict) else ("x".join(map(str, v)) if isinstance(v, tuple) else v))
 def test_overlapped_launches_bits(precision, box, kw, env):
     p, W, out = _box_params(box, **kw).replace(precision=precision), _field(box), []
@@ -52,3 +54,20 @@ def test_overlapped_adjoint_bits(box):
             out.append((g, J, dts, s.rhs_vjp(W), s.download_primitive()))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+# a single block of rows, a partial last one, several segments, rows shorter
+# than the window and a chunk, columns that are no multiple of eight
+@pytest.mark.parametrize("recon", ["WENO5", "MDCD", "UD7L", "LINEAR", "MDCD_HYBRID"])
+@pytest.mark.parametrize("box", [(33, 17, 9), (9, 130, 41), (500, 17, 18), (70, 75, 80)], ids=lambda b: "x".join(map(str, b)))
+def test_fp32_x_rows_bits(box, recon):
+    p = _box_params(box, fvs_type="LaxFriedrichs", recon=recon).replace(precision="fp32acc64")
+    W, out = _field(box), []
+    for rows in ("0", "1"):
+        with _solver(p, {"NS3D_XROWS": rows}) as s:
+            s.upload_primitive(W)
+            rhs = s.compute_rhs()
+            s.step(2)
+            out.append((rhs, s.download_primitive()))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
