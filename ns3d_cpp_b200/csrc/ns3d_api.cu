@@ -58,7 +58,8 @@ struct ns3d_ctx {
     // the z sweep fused with the stage update (NS3D_FUSE=1) or the two kernels
     // (NS3D_FUSE=0); the same bits either way
     bool fuse = false;
-    // FP64 small box: k_flux_small, T_acc as three separate terms (15 n values)
+    // FP64 small box: k_flux_small, T_acc as three separate terms (15 n values);
+    // false where they did not fit in device memory
     bool t3 = false;
     long long n = 0;
     double* wmem = nullptr;      // 3 state buffers x 6 arrays x n
@@ -871,7 +872,6 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
     const size_t n = (size_t)ctx->n;
     ctx->t3 = ctx->rsize == sizeof(double) && !ctx->fuse && !ctx->overlap && small_box(ctx->L);
     if (cudaMalloc(&ctx->wmem, sizeof(double) * 18 * n) != cudaSuccess ||
-        cudaMalloc(&ctx->tacc, ctx->rsize * (ctx->t3 ? 15 : 5) * n) != cudaSuccess ||
         cudaMalloc(&ctx->fv, ctx->rsize * (ctx->rsize == 4 ? fv_values_per_cell<float>() : fv_values_per_cell<double>()) * n) != cudaSuccess ||
         cudaMalloc(&ctx->ctrl, sizeof(Ctrl)) != cudaSuccess) {
         cudaGetLastError();
@@ -885,6 +885,17 @@ ns3d_status ns3d_create(const ns3d_params* p, int device, ns3d_ctx** out) {
         cudaMalloc(&ctx->step_times, sizeof(double) * kStepTimesCap0) != cudaSuccess)
         return bail(NS3D_ERR_NOMEM, "device allocation failed");
     ctx->step_times_cap = kStepTimesCap0;
+    // last: a device without room for the separate terms takes the marching
+    // kernels (the same bits), which need a third of the space
+    if (ctx->t3 && cudaMalloc(&ctx->tacc, ctx->rsize * 15 * n) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->tacc = nullptr;
+        ctx->t3 = false;
+    }
+    if (!ctx->t3 && cudaMalloc(&ctx->tacc, ctx->rsize * 5 * n) != cudaSuccess) {
+        cudaGetLastError();
+        return bail(NS3D_ERR_NOMEM, "device allocation failed");
+    }
     for (int b = 0; b < 3; ++b) ctx->slot[b] = ctx->wmem + (size_t)b * 6 * n;
     // a uniform quiescent state until the first upload (Field3D::allocate, :232-236)
     cudaMemsetAsync(ctx->wmem, 0, sizeof(double) * 18 * n, ctx->stream);

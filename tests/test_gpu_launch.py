@@ -71,3 +71,27 @@ def test_fp32_x_rows_bits(box, recon):
             out.append((rhs, s.download_primitive()))
     assert np.array_equal(out[0][0], out[1][0])
     assert np.array_equal(out[0][1], out[1][1])
+
+
+def test_small_box_context_without_room_for_the_separate_terms():
+    """A context of a box of k_flux_small takes 15 T_acc values a cell; where
+    the device has room for the 5 of the marching kernels only, it is created
+    with those and gives the same bits."""
+    import torch
+    box = (200, 150, 130)
+    n = box[0] * box[1] * box[2]
+    p, W, out, size = _box_params(box, fvs_type="LaxFriedrichs", recon="MDCD"), _field(box), [], []
+    hog = None
+    for room in (None, 8 * (18 + 9 + 10) * n):  # state, viscous fluxes, T_acc between the two
+        if room is not None:
+            torch.cuda.empty_cache()
+            hog = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+        with _solver(p, {}) as s:
+            s.upload_primitive(W)
+            s.step(2)
+            out.append(s.download_primitive())
+            size.append(s.device_bytes())
+    del hog
+    torch.cuda.empty_cache()
+    assert np.array_equal(*out)
+    assert size[0] - size[1] == 8 * 10 * n
