@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ns3d_adjoint.cuh"
 #include "ns3d_internal.h"
@@ -145,10 +146,10 @@ k_adj_face(DevParams P, StateView W, const double* __restrict__ lamR, double* __
 }
 
 // Gather of the split-flux cotangents of each cell and the transposed split
-// Jacobian: out(c) = (dF+/dw)^T lamF+(c) + (dF-/dw)^T lamF-(c).
+// Jacobian: lamW(c) += (dF+/dw)^T lamF+(c) + (dF-/dw)^T lamF-(c).
 template <int DIR, int FVS, int RC>
 __global__ void __launch_bounds__(128)
-k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __restrict__ out) {
+k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __restrict__ lamW) {
     constexpr int S = Stencil<RC>::S;
     constexpr int MID = (S - 1) / 2;
     // x: threads over j (G's x layout is j-fastest); y, z: threads over i
@@ -183,7 +184,7 @@ k_adj_cell(DevParams P, StateView W, const double* __restrict__ G, double* __res
     load_w5(W, id, w5);
     split_vjp<FVS, DIR>(w5, P.gamma, P.sw_eps, gp, gm, gw);
 #pragma unroll
-    for (int q = 0; q < 5; ++q) out[q * n + id] = gw[q];
+    for (int q = 0; q < 5; ++q) lamW[q * n + id] += gw[q];
 }
 
 // Viscous VJP, part 1: lam of the 12 gradients and the direct lam of u,v,w,T.
@@ -490,10 +491,11 @@ k_adj_stage(DevParams P, int stage, StateView Wk, StateView Wp, const double* la
     adj_stage_cell(P, stage, wk, Wp, id, lw, lamU0, lamR, lamWp, dt);
 }
 
-// lamW (the cotangent of state W so far) += the parts of k_adj_flux; finish:
+// lamW (the cotangent of state W so far) += the parts of k_adj_flux (PARTS; the
+// marching kernels have added theirs) and the second viscous part; finish:
 // lamW += (dU0/dW)^T lamU0 (W is a step's start state); next > 0: that stage's
 // adjoint, whose output state is W and whose input state is Wp, in place.
-template <int ORD>
+template <int ORD, bool PARTS>
 __global__ void __launch_bounds__(128)
 k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const double* __restrict__ lg,
              double* lamW, int finish, int next, StateView Wp, double* __restrict__ lamU0,
@@ -505,8 +507,10 @@ k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const doub
     const int i = (int)(id % P.nx), j = (int)(id / P.nx % P.ny), k = (int)(id / ((long long)P.nx * P.ny));
     double lw[5];
 #pragma unroll
-    for (int q = 0; q < 5; ++q)
-        lw[q] = ((lamW[q * n + id] + gw[q * n + id]) + gw[(5 + q) * n + id]) + gw[(10 + q) * n + id];
+    for (int q = 0; q < 5; ++q) {
+        lw[q] = lamW[q * n + id];
+        if constexpr (PARTS) lw[q] = ((lw[q] + gw[q * n + id]) + gw[(5 + q) * n + id]) + gw[(10 + q) * n + id];
+    }
     adj_visc2_cell<ORD>(P, W, lg, i, j, k, lw);
     double w5[5];
     if (finish || next) load_w5(W, id, w5);
@@ -524,7 +528,7 @@ k_adj_reduce(DevParams P, StateView W, const double* __restrict__ gw, const doub
     }
 }
 
-// The second viscous part alone, after the marching face kernels.
+// The first viscous part alone, after the marching face kernels.
 template <int ORD>
 __global__ void __launch_bounds__(128)
 k_adj_visc1(DevParams P, StateView W, const double* __restrict__ lamR, double* __restrict__ lg) {
@@ -551,7 +555,7 @@ k_adj_seed_ke(DevParams P, StateView W, double* __restrict__ lamW, double dV) {
 bool long_lines(const DevParams& P) { return P.nx > ADJ_NC || P.ny > ADJ_NC || P.nz > ADJ_NC; }
 
 template <int DIR, int FVS, int RC>
-cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw) {
+cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* lamW) {
     const DevParams& P = L.P;
     const int ext = DIR == 0 ? P.ny : P.nx;
     const int other = DIR == 2 ? P.ny : P.nz;
@@ -565,24 +569,25 @@ cudaError_t adj_dir(const LaunchCfg& L, StateView W, const double* lamR, double*
     const int cext = DIR == 0 ? P.ny : P.nx;
     const int tc = detail::threads_for(cext);
     const dim3 cg((cext + tc - 1) / tc, DIR == 0 ? P.nx : P.ny, P.nz);
-    k_adj_cell<DIR, FVS, RC><<<cg, tc, 0, L.stream>>>(P, W, G, gw + 5 * DIR * P.n);
+    k_adj_cell<DIR, FVS, RC><<<cg, tc, 0, L.stream>>>(P, W, G, lamW);
     return cudaGetLastError();
 }
 
-// G (long lines only): the window cotangents, 10 S blocks of n.
+// G: the three directions' parts (15 blocks of n) for k_adj_reduce; for long
+// lines the window cotangents (10 S blocks), whose sums are added to lamW here.
 template <int FVS, int RC>
-cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw, double* lg) {
+cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* lg, double* lamW) {
     const DevParams& P = L.P;
     if (!long_lines(P)) {
         // 128 to 256 cells a block: several blocks per SM, at least two per SM for each direction
         const long long target = std::min(256ll, std::max(64ll, 3 * P.n / (2 * 148)));
         const SmallShape sh = small_shape(P, target, ADJ_NC, ADJ_T);
         return launch_pdl(L, k_adj_flux<FVS, RC>, small_blocks(sh), ADJ_T, adj_smem<RC>(small_cells(P, sh)), P, W,
-                          lamR, gw, lg, sh);
+                          lamR, G, lg, sh);
     }
-    cudaError_t e = adj_dir<0, FVS, RC>(L, W, lamR, G, gw);
-    if (e == cudaSuccess) e = adj_dir<1, FVS, RC>(L, W, lamR, G, gw);
-    if (e == cudaSuccess) e = adj_dir<2, FVS, RC>(L, W, lamR, G, gw);
+    cudaError_t e = adj_dir<0, FVS, RC>(L, W, lamR, G, lamW);
+    if (e == cudaSuccess) e = adj_dir<1, FVS, RC>(L, W, lamR, G, lamW);
+    if (e == cudaSuccess) e = adj_dir<2, FVS, RC>(L, W, lamR, G, lamW);
     if (e != cudaSuccess) return e;
     const int th = detail::threads_for(P.nx);
     const dim3 g = detail::cell_grid(P, th);
@@ -593,12 +598,12 @@ cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double
 }
 
 template <int FVS>
-cudaError_t adj_flux_rc(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* gw, double* lg) {
+cudaError_t adj_flux_rc(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* lg, double* lamW) {
     switch (L.rc) {
-    case RC_WENO5: return adj_flux<FVS, RC_WENO5>(L, W, lamR, G, gw, lg);
-    case RC_LINEAR: return adj_flux<FVS, RC_LINEAR>(L, W, lamR, G, gw, lg);
-    case RC_LIN6: return adj_flux<FVS, RC_LIN6>(L, W, lamR, G, gw, lg);
-    case RC_LIN8: return adj_flux<FVS, RC_LIN8>(L, W, lamR, G, gw, lg);
+    case RC_WENO5: return adj_flux<FVS, RC_WENO5>(L, W, lamR, G, lg, lamW);
+    case RC_LINEAR: return adj_flux<FVS, RC_LINEAR>(L, W, lamR, G, lg, lamW);
+    case RC_LIN6: return adj_flux<FVS, RC_LIN6>(L, W, lamR, G, lg, lamW);
+    case RC_LIN8: return adj_flux<FVS, RC_LIN8>(L, W, lamR, G, lg, lamW);
     default: return cudaErrorNotSupported;
     }
 }
@@ -608,7 +613,7 @@ cudaError_t adj_flux_rc(const LaunchCfg& L, StateView W, const double* lamR, dou
 int adj_scratch_blocks(const LaunchCfg& L) {
     if (!long_lines(L.P)) return 15;
     const int S = L.rc == RC_LIN8 ? 8 : (L.rc == RC_LINEAR ? 2 : 6);
-    return 15 + 2 * S * 5;
+    return 2 * S * 5;
 }
 
 int adj_rhs_vjp_launches(const LaunchCfg& L) { return long_lines(L.P) ? 8 : 2; }
@@ -616,18 +621,20 @@ int adj_rhs_vjp_launches(const LaunchCfg& L) { return long_lines(L.P) ? 8 : 2; }
 cudaError_t adj_rhs_vjp(const LaunchCfg& L, StateView W, double* G, double* lg, double* lamW, int finish, int next,
                         StateView Wp, double* lamU0, double* lamR, double dt) {
     const DevParams& P = L.P;
-    double* gw = G;
-    double* Gw = G + 15 * P.n;
-    cudaError_t e = L.fvs == FV_SW ? adj_flux_rc<FV_SW>(L, W, lamR, Gw, gw, lg)
-                                   : adj_flux_rc<FV_LF>(L, W, lamR, Gw, gw, lg);
+    cudaError_t e = L.fvs == FV_SW ? adj_flux_rc<FV_SW>(L, W, lamR, G, lg, lamW)
+                                   : adj_flux_rc<FV_LF>(L, W, lamR, G, lg, lamW);
     if (e != cudaSuccess) return e;
     const unsigned b = (unsigned)((P.n + 127) / 128);
-    auto reduce = [&](auto kernel) {
-        return launch_pdl(L, kernel, b, 128, 0, P, W, gw, lg, lamW, finish, next, Wp, lamU0, lamR, dt);
+    auto reduce = [&](auto parts) {
+        constexpr bool PARTS = decltype(parts)::value;
+        auto go = [&](auto kernel) {
+            return launch_pdl(L, kernel, b, 128, 0, P, W, G, lg, lamW, finish, next, Wp, lamU0, lamR, dt);
+        };
+        if (P.vis_order == 4) return go(k_adj_reduce<4, PARTS>);
+        if (P.vis_order == 6) return go(k_adj_reduce<6, PARTS>);
+        return go(k_adj_reduce<8, PARTS>);
     };
-    if (P.vis_order == 4) return reduce(k_adj_reduce<4>);
-    if (P.vis_order == 6) return reduce(k_adj_reduce<6>);
-    return reduce(k_adj_reduce<8>);
+    return long_lines(P) ? reduce(std::false_type{}) : reduce(std::true_type{});
 }
 
 cudaError_t adj_stage(const LaunchCfg& L, int stage, StateView Wk, StateView Wp, const double* lamWk, double* lamU0,

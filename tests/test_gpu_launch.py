@@ -95,3 +95,16 @@ def test_small_box_context_without_room_for_the_separate_terms():
     torch.cuda.empty_cache()
     assert np.array_equal(*out)
     assert size[0] - size[1] == 8 * 10 * n
+
+
+@pytest.mark.parametrize("kw,S", [(dict(), 6), (dict(recon="UD7L"), 8)], ids=["WENO5", "UD7L"])
+def test_adjoint_scratch_of_long_lines(kw, S):
+    """A right-hand side's VJP with a line above 300 cells keeps, per cell, the
+    cotangents in and out (5 each), the windows' (2 S 5) and the viscous ones (16)."""
+    box = (304, 10, 9)
+    p, W = _box_params(box, **kw), _field(box)
+    with _solver(p, {}) as s:
+        s.upload_primitive(W)
+        before = s.device_bytes()
+        s.rhs_vjp(W)
+        assert s.device_bytes() - before == 8 * (5 + 5 + 10 * S + 16) * 304 * 10 * 9
