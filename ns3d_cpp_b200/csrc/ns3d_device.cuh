@@ -71,8 +71,9 @@ inline void derive_quotients(DevParams& P) {
 // With y from rcp_cubic(b) instead of the rounded reciprocal, q is still within
 // an ulp or so and r still exact, and what is rounded last, q + r y, differs
 // from a/b by r times y's error: at most 2^-104 of it. So the result is RN(a/b)
-// unless a/b lies within 2^-104 of a rounding midpoint (about one random
-// operand pair in 2^51).
+// unless a/b lies within 2^-104 of a rounding midpoint: about one random
+// operand pair in 2^51, and every power of two over a b whose significand is all
+// ones (1 - 2^-53, a density one rounding below 1): divisor_ok() keeps such b away.
 __device__ __forceinline__ double div_rcp(double a, double b, double y) {
     const double q = a * y;
     const double r = fma(-b, q, a);
@@ -110,15 +111,20 @@ __device__ __forceinline__ double sqrt_cubic(double b) {
 __device__ __forceinline__ bool mid_range(double x) {
     return (unsigned)(__double2hiint(x) - ((1023 - 900) << 20)) < (1800u << 20);
 }
+// A divisor for rcp_cubic and div_rcp: mid-range, its low 32 bits not all ones
+// (see div_rcp).
+__device__ __forceinline__ bool divisor_ok(double b) {
+    return mid_range(b) && (unsigned)__double2loint(b) != 0xffffffffu;
+}
 __device__ __forceinline__ bool finite_hi(double x) {
     return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
-// a / b: div_rcp where its range allows (b mid-range, quotient finite), else
+// a / b: div_rcp where its range allows (divisor_ok, quotient finite), else
 // the compiler's division out of line.
 static __device__ __noinline__ double div_cold(double a, double b) { return a / b; }
 __device__ __forceinline__ double quot_mid(double a, double b) {
     const double q = div_rcp(a, b, rcp_cubic(b));
-    return mid_range(b) && finite_hi(q) ? q : div_cold(a, b);
+    return divisor_ok(b) && finite_hi(q) ? q : div_cold(a, b);
 }
 static __device__ __noinline__ double sqrt_cold(double b) { return sqrt(b); }
 __device__ __forceinline__ double sqrt_mid(double b) {
@@ -179,7 +185,7 @@ __device__ __forceinline__ double get_mu_exact(double T, double mu_ref, double S
     const double p15 = p + (e + 0.5 * (r * s));
     const double TS = T + S;
     const double q = div_rcp(mu_ref * p15 * (1.0 + S), TS, rcp_cubic(TS));
-    if (mid_range(T) && mid_range(TS) && finite_hi(q)) return q;
+    if (mid_range(T) && divisor_ok(TS) && finite_hi(q)) return q;
     return get_mu_cold(T, mu_ref, S);
 }
 
@@ -294,7 +300,7 @@ __device__ __noinline__ void split_ieee_cold(double gamma, double eps, const dou
 // constant's), the products with the zero components of the normal left out
 // (they add a zero) and 0.5 (l +- |l|) as the selection it is. States outside
 // the ranges those need take split_ieee: density, pressure or sound speed extreme or not
-// a number, energy not finite.
+// a number, density no divisor_ok(), energy not finite.
 template <int FVS, int N1, int N2, int N3>
 __device__ __forceinline__ void split_exact(const DevParams& P, const double* raw,
                                             double Fp[5], double Fm[5]) {
@@ -310,7 +316,7 @@ __device__ __forceinline__ void split_exact(const DevParams& P, const double* ra
     const double E = rho * (div_rcp(p, g1r, rcp_cubic(g1r)) + kinetic);
     const double c = sqrt_cubic(c2);
     const double un = N1 ? u : (N2 ? v : w);
-    bool ok = mid_range(rho) && mid_range(p) && mid_range(c2) && finite_hi(E);
+    bool ok = divisor_ok(rho) && mid_range(p) && mid_range(c2) && finite_hi(E);
     if constexpr (FVS == FV_SW) {
         const double l1 = un - c, l2 = un, l3 = un + c;
         double l1p, l1m, l2p, l2m, l3p, l3m;

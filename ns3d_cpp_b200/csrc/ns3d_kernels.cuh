@@ -1537,7 +1537,7 @@ __device__ __forceinline__ void stage_apply(const DevParams& P, const double U0[
         v = div_rcp(U[2], rr, yr);
         w = div_rcp(U[3], rr, yr);
         double e = div_rcp(U[4], rr, yr);
-        if (!mid_range(rr) || !finite_hi(u) || !finite_hi(v) || !finite_hi(w) || !finite_hi(e)) {
+        if (!divisor_ok(rr) || !finite_hi(u) || !finite_hi(v) || !finite_hi(w) || !finite_hi(e)) {
             u = div_cold(U[1], rr);
             v = div_cold(U[2], rr);
             w = div_cold(U[3], rr);
