@@ -39,10 +39,10 @@ struct DevParams {
     double mdcd_disp, mdcd_diss;
     int vis_order;   // 4, 6, 8
     int pdl;         // 1: the launches overlap (launch_pdl, pdl_enter)
-    // divisors of the central derivatives (12 h, 60 h or h) along x, y, z, and
-    // the reciprocals RN(1/b) of these, of the heat flux's Pr and of the
-    // split's 2 gamma (see quot_rcp)
-    double dd[3], rdd[3], rPr, r2g;
+    // divisors of the central derivatives (12 h, 60 h or h) along x, y, z times
+    // 2^54, and the reciprocals RN(1/b) of the divisors (also times 2^-54), of the
+    // heat flux's Pr and of the split's 2 gamma (see quot_wide, quot_rcp)
+    double dd54[3], rdd[3], rdd54[3], rPr, r2g;
 };
 
 // The derived constants above, from the fields before them.
@@ -50,8 +50,10 @@ inline void derive_quotients(DevParams& P) {
     const double c = P.vis_order == 4 ? 12.0 : (P.vis_order == 6 ? 60.0 : 1.0);
     const double h[3] = {P.dx, P.dy, P.dz};
     for (int d = 0; d < 3; ++d) {
-        P.dd[d] = c * h[d];
-        P.rdd[d] = 1.0 / P.dd[d];
+        const double b = c * h[d];
+        P.dd54[d] = b * 0x1p54;
+        P.rdd[d] = 1.0 / b;
+        P.rdd54[d] = P.rdd[d] * 0x1p-54;
     }
     P.rPr = 1.0 / P.Pr;
     P.r2g = 1.0 / (2.0 * P.gamma);
@@ -66,7 +68,9 @@ inline void derive_quotients(DevParams& P) {
 // -- if y is 1/b correctly rounded and q is within one ulp of a/b, then
 // r = a - b q is a double (one exact FMA) and RN(q + r y) = RN(a/b). Here
 // q = RN(a y) is within one ulp, so the result equals the IEEE quotient a / b
-// bit for bit (finite a/b in the normal range), in three operations.
+// bit for bit, in three operations, where b > 0 (the residual is formed with the
+// other sign, so that a zero keeps its own: -0 / b is -0), |a| is zero or above
+// 2^-960 (below that the residual is no double) and a/b finite and normal.
 //
 // With y from rcp_cubic(b) instead of the rounded reciprocal, q is still within
 // an ulp or so and r still exact, and what is rounded last, q + r y, differs
@@ -76,8 +80,18 @@ inline void derive_quotients(DevParams& P) {
 // ones (1 - 2^-53, a density one rounding below 1): divisor_ok() keeps such b away.
 __device__ __forceinline__ double div_rcp(double a, double b, double y) {
     const double q = a * y;
-    const double r = fma(-b, q, a);
-    return fma(r, y, q);
+    const double r = fma(b, q, -a);
+    return fma(-r, y, q);
+}
+
+// div_rcp without its lower limit: the residual is formed 2^54 times as large,
+// from b54 = 2^54 b and a product more, and y54 = 2^-54 y takes that back (a
+// subnormal quotient can miss a tie, by its last place). For |a| up to 2^969; a
+// larger one gives no finite value.
+__device__ __forceinline__ double div_wide(double a, double b54, double y, double y54) {
+    const double q = a * y;
+    const double r = fma(b54, q, -(a * 0x1p54));
+    return fma(-r, y54, q);
 }
 
 // 1/b within an ulp for b in the normal range whose reciprocal is normal: the
@@ -92,7 +106,7 @@ __device__ __forceinline__ double rcp_cubic(double b) {
     return fma(x, fma(e, e, e), x);
 }
 
-// sqrt(b) for b in [2^-900, 2^900]: the estimate y0 of 1/sqrt b (about 2^-20),
+// sqrt(b) for b of mid_range(): the estimate y0 of 1/sqrt b (about 2^-20),
 // one third-order step y = y0 (1 + e/2 + 3 e^2/8), e = 1 - b y0^2, and the
 // final correction s + (b - s^2) y / 2 with the residual exact (one FMA), which
 // leaves 2^-104 before the last rounding: RN(sqrt b) as in div_rcp's note
@@ -106,10 +120,11 @@ __device__ __forceinline__ double sqrt_cubic(double b) {
     return fma(fma(-s, s, b), 0.5 * y, s);
 }
 
-// x in [2^-900, 2^900): the range in which rcp_cubic, div_rcp and sqrt_cubic
-// neither overflow nor lose a residual to underflow (sign or NaN: false).
+// x in [2^-480, 2^480) (sign or NaN: false): with a dividend and a divisor of this
+// range rcp_cubic, div_rcp and sqrt_cubic neither overflow nor lose a residual
+// or a quotient to underflow.
 __device__ __forceinline__ bool mid_range(double x) {
-    return (unsigned)(__double2hiint(x) - ((1023 - 900) << 20)) < (1800u << 20);
+    return (unsigned)(__double2hiint(x) - ((1023 - 480) << 20)) < (960u << 20);
 }
 // A divisor for rcp_cubic and div_rcp: mid-range, its low 32 bits not all ones
 // (see div_rcp).
@@ -119,12 +134,12 @@ __device__ __forceinline__ bool divisor_ok(double b) {
 __device__ __forceinline__ bool finite_hi(double x) {
     return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
-// a / b: div_rcp where its range allows (divisor_ok, quotient finite), else
-// the compiler's division out of line.
+// a / b: div_rcp where its range allows (divisor_ok, a mid-range), else the compiler's
+// division out of line.
 static __device__ __noinline__ double div_cold(double a, double b) { return a / b; }
 __device__ __forceinline__ double quot_mid(double a, double b) {
     const double q = div_rcp(a, b, rcp_cubic(b));
-    return divisor_ok(b) && finite_hi(q) ? q : div_cold(a, b);
+    return divisor_ok(b) && mid_range(a) ? q : div_cold(a, b);
 }
 static __device__ __noinline__ double sqrt_cold(double b) { return sqrt(b); }
 __device__ __forceinline__ double sqrt_mid(double b) {
@@ -136,8 +151,15 @@ __device__ __forceinline__ double sqrt_mid(double b) {
 // and NaN of the IEEE quotient (its residual would turn them into NaN).
 __device__ __forceinline__ double quot_rcp(double a, double b, double y) {
     const double q = a * y;
-    const double r = fma(fma(-b, q, a), y, q);
+    const double r = div_rcp(a, b, y);
     return finite_hi(q) ? r : q;
+}
+// The same by div_wide, for quotients that may be of any size (a derivative in the
+// far tail of a disturbance); |a| above 2^969: a y, within an ulp (a second
+// correction there cost k_update 16%, 1000 -> 1164 us at 256^3).
+__device__ __forceinline__ double quot_wide(double a, double b54, double y, double y54) {
+    const double r = div_wide(a, b54, y, y54);
+    return finite_hi(r) ? r : a * y;
 }
 
 // ---------------------------------------------------------------------------
@@ -907,7 +929,7 @@ __device__ __forceinline__ R dcentral(F f, R h) {
 }
 
 // The same derivative along x, y or z (dir 0, 1, 2; spacing h) of a box: the FP64 form's
-// division by the constant divisor as quot_rcp (the IEEE quotient; twelve per
+// division by the constant divisor as quot_wide (the IEEE quotient; twelve per
 // cell in the viscous flux and twelve in its divergence).
 template <class R, int ORD, class F>
 __device__ __forceinline__ R dcentral_dir(const DevParams& P, int dir, F f, R h) {
@@ -922,7 +944,7 @@ __device__ __forceinline__ R dcentral_dir(const DevParams& P, int dir, F f, R h)
             const double c1 = 0.8, c2 = -0.2, c3 = 0.0380952380952381, c4 = -0.00357142857142857;
             x = c1 * (f(1) - f(-1)) + c2 * (f(2) - f(-2)) + c3 * (f(3) - f(-3)) + c4 * (f(4) - f(-4));
         }
-        return quot_rcp(x, P.dd[dir], P.rdd[dir]);
+        return quot_wide(x, P.dd54[dir], P.rdd[dir], P.rdd54[dir]);
     } else {
         return dcentral<R, ORD>(f, h);
     }

@@ -1531,13 +1531,13 @@ __device__ __forceinline__ void stage_apply(const DevParams& P, const double U0[
         p = (gamma - 1.0) * (U[4] - rr * (0.5 * (u * u + v * v + w * w)));
         T = p * ir * (1.0 / P.Rgas);
     } else {
-        // U / rr by one reciprocal (the IEEE quotients, see div_rcp)
-        const double yr = rcp_cubic(rr);
-        u = div_rcp(U[1], rr, yr);
-        v = div_rcp(U[2], rr, yr);
-        w = div_rcp(U[3], rr, yr);
+        // U / rr by one reciprocal (the IEEE quotients, see div_wide)
+        const double yr = rcp_cubic(rr), yr54 = yr * 0x1p-54, rr54 = rr * 0x1p54;
+        u = div_wide(U[1], rr54, yr, yr54);
+        v = div_wide(U[2], rr54, yr, yr54);
+        w = div_wide(U[3], rr54, yr, yr54);
         double e = div_rcp(U[4], rr, yr);
-        if (!divisor_ok(rr) || !finite_hi(u) || !finite_hi(v) || !finite_hi(w) || !finite_hi(e)) {
+        if (!divisor_ok(rr) || !finite_hi(u) || !finite_hi(v) || !finite_hi(w) || !mid_range(e)) {
             u = div_cold(U[1], rr);
             v = div_cold(U[2], rr);
             w = div_cold(U[3], rr);
