@@ -637,8 +637,9 @@ __device__ __forceinline__ R weno5_ieee(R f0, R f1, R f2, R f3, R f4) {
 //   * an FMA wherever one factor is a power of two (the product is exact, so
 //     the FMA rounds what the separate operations round once).
 // A reciprocal whose argument overflowed gives NaN where the IEEE quotient is
-// 0: callers test the face for non-finite values and recompute it with
-// weno5_ieee (see recon_face).
+// 0, and alpha_k of a window that varies by 2^240 or more are too small for
+// div_rcp: callers test the face for values that are not finite or that large
+// and recompute it with weno5_ieee (see recon_face).
 __device__ __forceinline__ double weno5(double f0, double f1, double f2, double f3, double f4) {
     const double eps = 1e-6;
     const double m3 = 3.0 * f2;
@@ -806,13 +807,15 @@ __device__ __forceinline__ R mdcd_hybrid(const R* s, const R* lin6, R disp, R di
     return (aa0 * q0 + aa1 * q1 + aa2 * q2 + aa3 * q3) / (aa0 + aa1 + aa2 + aa3);
 }
 
-// Whether any of a face's five values is infinite or NaN (integer tests: the
-// FP64 pipe is what bounds the callers).
-__device__ __forceinline__ bool any_nonfinite(const double* a) {
+// Whether a face value is infinite, NaN or beyond 2^200 (integer tests: the FP64
+// pipe is what bounds the callers), and whether any of a face's five is.
+constexpr int FACE_HUGE = (1023 + 200) << 20;
+__device__ __forceinline__ bool face_huge(double a) { return (__double2hiint(a) & 0x7fffffff) >= FACE_HUGE; }
+__device__ __forceinline__ bool any_huge(const double* a) {
     int m = 0;
 #pragma unroll
     for (int q = 0; q < 5; ++q) m = max(m, __double2hiint(a[q]) & 0x7fffffff);
-    return m >= 0x7ff00000;
+    return m >= FACE_HUGE;
 }
 
 // One reconstruction of a window s[0..S-1] (already oriented).
@@ -833,17 +836,13 @@ __device__ __forceinline__ R reconstruct(const R* s, const R* lin, R disp, R dis
     }
 }
 
-// The face values of the five components from their windows: P(m, q) / M(m, q)
-// return component q at window position m of F+ / of F- (reversed already, as
-// reconstruct_select does for flag < 0). FP64 WENO5: the branch-free form, and
-// once more by weno5_ieee when a value comes out infinite or NaN, so that
-// overflowing windows give what the IEEE divisions give (a window that holds
-// an infinity is NaN either way). DYN: P and M take a loop variable there (a
-// window in shared memory; one in registers needs q at compile time).
+// FP64 WENO5: the five values once more by weno5_ieee when one comes out infinite,
+// NaN or huge, so that windows beyond weno5's range give what the IEEE divisions give (a
+// window that holds an infinity is NaN either way). P, M, DYN: see recon_face.
 template <class R, int RC, bool DYN, class GP, class GM>
-__device__ __forceinline__ void recon_face_nonfinite(GP P, GM M, R face[5]) {
+__device__ __forceinline__ void recon_face_huge(GP P, GM M, R face[5]) {
     if constexpr (sizeof(R) == 8 && RC == RC_WENO5) {
-        if (any_nonfinite(face)) {
+        if (any_huge(face)) {
 #pragma unroll(DYN ? 1 : 5)
             for (int q = 0; q < 5; ++q) {
                 const R f = weno5_ieee<R>(P(0, q), P(1, q), P(2, q), P(3, q), P(4, q)) +
@@ -858,6 +857,10 @@ __device__ __forceinline__ void recon_face_nonfinite(GP P, GM M, R face[5]) {
     }
 }
 
+// The face values of the five components from their windows: P(m, q) / M(m, q)
+// return component q at window position m of F+ / of F- (reversed already, as
+// reconstruct_select does for flag < 0). DYN: P and M take a loop variable in
+// recon_face_huge (a window in shared memory; one in registers needs q at compile time).
 template <class R, int RC, bool DYN, class GP, class GM>
 __device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R diss, R face[5]) {
     constexpr int S = Stencil<RC>::S;
@@ -873,7 +876,7 @@ __device__ __forceinline__ void recon_face(GP P, GM M, const R* lin, R disp, R d
         const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
         face[q] = plus_face + minus_face;
     }
-    recon_face_nonfinite<R, RC, DYN>(P, M, face);
+    recon_face_huge<R, RC, DYN>(P, M, face);
 }
 
 // recon_face of the FP64 form from 16-byte words: X(m, k) is word k of window

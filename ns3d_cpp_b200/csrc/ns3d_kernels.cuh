@@ -117,7 +117,7 @@ __device__ __forceinline__ void char_face(double gamma, const double* wl, const 
         const R minus_face = reconstruct<R, RC>(b, lin, disp, diss);
         wc[q] = plus_face + minus_face;
         if constexpr (sizeof(R) == 8 && RC == RC_WENO5) {  // as in recon_face
-            if ((__double2hiint(wc[q]) & 0x7ff00000) == 0x7ff00000)
+            if (face_huge(wc[q]))
                 wc[q] = weno5_ieee<R>(a[0], a[1], a[2], a[3], a[4]) +
                         weno5_ieee<R>(b[0], b[1], b[2], b[3], b[4]);
         }
@@ -678,7 +678,7 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
             auto M = [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); };
             if constexpr (sizeof(R) == 8) {
                 recon_words<RC>([&](int m, int k) { return ring.a[wq][k][cell[m]]; }, lin, disp, diss, face);
-                recon_face_nonfinite<R, RC, true>(P, M, face);
+                recon_face_huge<R, RC, true>(P, M, face);
             } else {
                 recon_face<R, RC, true>(P, M, lin, disp, diss, face);
             }
@@ -1769,7 +1769,7 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
                 auto M = [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); };
                 if constexpr (sizeof(R) == 8) {
                     recon_words<RC>([&](int m, int k) { return ring.a[sl[m]][k][tid]; }, lin, disp, diss, face);
-                    recon_face_nonfinite<R, RC, true>(P, M, face);
+                    recon_face_huge<R, RC, true>(P, M, face);
                 } else {
                     recon_face<R, RC, true>(P, M, lin, disp, diss, face);
                 }

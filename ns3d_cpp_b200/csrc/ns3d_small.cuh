@@ -109,7 +109,7 @@ constexpr int small_most(bool chr) { return chr ? 300 : SMALL_NC; }
 constexpr int small_smem(int nc, bool chr) { return nc * small_doubles(chr) * (int)sizeof(double); }
 
 // char_face with everything by the general code, for faces whose values come
-// out infinite or NaN below.
+// out infinite, NaN or huge below.
 template <int DIR, int RC>
 __device__ __noinline__ void char_face_cold(const DevParams& P, const double* wl, const double* wr,
                                             const double* F, int nc, const int* w, double* face) {
@@ -248,7 +248,7 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
             for (int m = 0; m < S; ++m) w[m] = tl.at(s - MID + m) + l * tl.cl;
             double face[5];
             char_face_fast<DIR, RC>(P, F, g, nc, w, face);
-            if (any_nonfinite(face)) {
+            if (any_huge(face)) {
                 double wl[5], wr[5], fc[5];
                 int wi[S];
                 const long long il = tl.id(l, s), ir = tl.id(l, s + 1 == tl.len ? 0 : s + 1);
@@ -286,10 +286,11 @@ __device__ __forceinline__ void small_sweep(const DevParams& P, const StateView&
                     a[m] = fp[w[m]];
                     bm[S - 1 - m] = fm[w[m]];  // reconstruct_select reverses for flag < 0
                 }
-                double f = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss) +
-                           reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
-                if constexpr (RC == RC_WENO5) {  // as in recon_face
-                    if (!finite_hi(f))
+                const double rp = reconstruct<double, RC>(a, P.lin, P.mdcd_disp, P.mdcd_diss);
+                const double rm = reconstruct<double, RC>(bm, P.lin, P.mdcd_disp, P.mdcd_diss);
+                double f = rp + rm;
+                if constexpr (RC == RC_WENO5) {  // as in recon_face (the two may cancel)
+                    if (face_huge(rp) || face_huge(rm))
                         f = weno5_ieee<double>(a[0], a[1], a[2], a[3], a[4]) +
                             weno5_ieee<double>(bm[0], bm[1], bm[2], bm[3], bm[4]);
                 }

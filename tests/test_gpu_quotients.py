@@ -9,7 +9,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from conftest import ROOT, ref_cfg
+from conftest import ROOT, ref_cfg, scheme_id
 from test_gpu_parity import params_from_cfg
 from test_gpu_routes import _solver
 
@@ -164,3 +164,22 @@ def test_velocities_of_any_size_match_oracle(oracle_mod, scale, small):
         got = s.download_primitive()
     for q in range(5):
         assert np.array_equal(got[q].view(np.uint64), np.ascontiguousarray(want[q]).view(np.uint64)), q
+
+
+@pytest.mark.parametrize("small", ["0", "10000000"], ids=["marching", "small"])
+@pytest.mark.parametrize("kw", [dict(), dict(fvs_type="LaxFriedrichs"), dict(char_recon="true")], ids=scheme_id)
+def test_windows_that_vary_hugely_match_oracle(oracle_mod, kw, small):
+    """WENO5 windows that vary by 2^240 and more, whose weights' terms are too small
+    for the branch-free quotients: the mass equation (no T^1.5) has the oracle's bits."""
+    n = 16
+    cfg = ref_cfg(n, **kw)
+    r = np.random.default_rng(3)
+    W = np.empty((5, n, n, n))
+    W[0] = 1.0 + 0.1 * r.random((n, n, n))
+    W[1:4] = r.standard_normal((3, n, n, n))
+    W[4] = 10.0 ** r.uniform(140, 156, (n, n, n))  # split mass fluxes of rho c
+    want = oracle_mod.Oracle(cfg).rhs(W)
+    with _solver(params_from_cfg(cfg), {"NS3D_SMALL": small}) as s:
+        s.upload_primitive(W)
+        got = s.compute_rhs()
+    assert np.array_equal(got[0], want[0], equal_nan=True)
