@@ -264,7 +264,10 @@ ns3d_status ns3d_compute_rhs_noalloc(const ns3d_params *p, const double *rho, co
 
 /* ---- instrumentation (no reference counterpart) -------------------------- */
 
-/* Kernel classes timed by ns3d_profile. */
+/* Kernel classes timed by ns3d_profile. FP64 boxes whose fluxes run as one launch
+ * (k_flux_small: all sweeps and the viscous flux side by side) book that launch
+ * under NS3D_KERNEL_OTHER, with the loop's control; SWEEP_X, _Y, _Z and VISC_FLUX
+ * then count no launches. */
 enum {
     NS3D_KERNEL_SWEEP_X = 0, NS3D_KERNEL_SWEEP_Y = 1, NS3D_KERNEL_SWEEP_Z = 2,
     NS3D_KERNEL_VISC_FLUX = 3, NS3D_KERNEL_UPDATE = 4, NS3D_KERNEL_OTHER = 5,

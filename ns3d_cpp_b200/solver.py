@@ -335,6 +335,9 @@ class Solver:
         self._ck(self.lib.ns3d_profile(self.ctx, int(bool(enable))))
 
     def profile_read(self) -> dict:
+        """{class: (device ms, launches)} since profile(True). FP64 boxes whose
+        fluxes run as one launch have it under "other"; their sweep and viscous
+        classes count no launches."""
         ms = (ctypes.c_double * len(self.KERNEL_CLASSES))()
         n = (ctypes.c_longlong * len(self.KERNEL_CLASSES))()
         self._ck(self.lib.ns3d_profile_read(self.ctx, ms, n))

@@ -61,7 +61,20 @@ def _kernel_bytes(cls: str, rsize: int) -> float:
     return {"sweep_x": w + 5 * rsize, "sweep_y": w + 10 * rsize, "sweep_z": w + 10 * rsize,
             "visc_flux": 32 + fv * rsize,
             "update": (5.0 / 3.0) * w + (5 + fv) * rsize + 48,  # stage 1 reads one state
-            "sweep_z_update": (5.0 / 3.0) * w + (5 + fv) * rsize + 48}.get(cls, 0.0)
+            "sweep_z_update": (5.0 / 3.0) * w + (5 + fv) * rsize + 48,
+            # the three sweeps' states and terms and the viscous flux in one launch
+            "fluxes": 3 * (w + 5 * rsize) + 32 + fv * rsize}.get(cls, 0.0)
+
+
+def _one_launch_fluxes(prof: dict) -> dict:
+    """profile_read()'s classes with the one-launch fluxes of a small FP64 box, which
+    the library books under "other" with the control launches and the monitors, as a
+    class of their own: as many launches as updates, and all of that class's time."""
+    if prof["sweep_x"][1] or not prof["update"][1]:
+        return prof
+    prof = dict(prof)
+    prof["fluxes"] = (prof.pop("other")[0], prof["update"][1])
+    return prof
 
 
 def params_for(w: dict, recon: str, precision: str, dt_fixed: float = -1.0) -> SolverParams:
@@ -122,7 +135,7 @@ def run_one(w: dict, W: np.ndarray, recon: str, precision: str, steps: int, devi
                            mach_t=st["mach_t"], u_rms=st["u_rms"])
                 mon["spectrum_head"] = [float(x) for x in s.compute_energy_spectrum(12)]
             out["monitors"].append(mon)
-        prof = s.profile_read()
+        prof = _one_launch_fluxes(s.profile_read())
         s.profile(False)
         out["final_spectrum"] = [float(x) for x in s.compute_energy_spectrum()]
     peak = _peak_gbs()

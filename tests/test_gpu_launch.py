@@ -108,3 +108,13 @@ def test_adjoint_scratch_of_long_lines(kw, S):
         before = s.device_bytes()
         s.rhs_vjp(W)
         assert s.device_bytes() - before == 8 * (5 + 5 + 10 * S + 16) * 304 * 10 * 9
+
+
+def test_workload_reports_the_one_launch_fluxes():
+    """The library books them under "other"; the workload runner lists them with
+    their bandwidth, as it does the sweeps of larger boxes."""
+    from ns3d_cpp_b200 import workloads
+    w = workloads.WORKLOADS["tgv32"]
+    k = workloads.run_one(w, workloads.initial_for(w), "weno5", "fp64", 4, 0)["kernels"]
+    assert k["fluxes"]["launches"] == k["update"]["launches"] == 12 and k["fluxes"]["hbm_frac"] > 0
+    assert "sweep_x" not in k and "other" not in k
