@@ -579,7 +579,9 @@ template <int FVS, int RC>
 cudaError_t adj_flux(const LaunchCfg& L, StateView W, const double* lamR, double* G, double* lg, double* lamW) {
     const DevParams& P = L.P;
     if (!long_lines(P)) {
-        // 128 to 256 cells a block: several blocks per SM, at least two per SM for each direction
+        // 64 to 256 cells a block, as in flux_small. With one line a block along y and z
+        // (extents above 150) still faster than the marching kernels: a VJP's kernels,
+        // WENO5, 200^3 12.8 -> 6.7 ms, 256^3 22.2 -> 13.0, 40x300x300 6.6 -> 2.9
         const long long target = std::min(256ll, std::max(64ll, 3 * P.n / (2 * 148)));
         const SmallShape sh = small_shape(P, target, ADJ_NC, ADJ_T);
         return launch_pdl(L, k_adj_flux<FVS, RC>, small_blocks(sh), ADJ_T, adj_smem<RC>(small_cells(P, sh)), P, W,

@@ -43,9 +43,9 @@ struct DevParams {
     // 2^54, and the reciprocals RN(1/b) of the divisors (also times 2^-54), of the
     // heat flux's Pr and of the split's 2 gamma (see quot_wide, quot_rcp)
     double dd54[3], rdd[3], rdd54[3], rPr, r2g;
-    // without it k_update<float, 8> spills 32 bytes instead of 16 (a step at 256^3
-    // 6735 -> 6860 us; where a kernel's later arguments lie in the parameter block
-    // decides: 16 n + 8 bytes more than without the constants above is the bad size)
+    // keeps the block's size a multiple of 16 bytes: without it k_update<float, 8>
+    // spills 32 bytes instead of 16 (a step at 256^3 6735 -> 6860 us; alignas(16) in its
+    // place 6832)
     double pad;
 };
 

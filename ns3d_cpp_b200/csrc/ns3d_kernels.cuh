@@ -674,13 +674,13 @@ __device__ __forceinline__ void x_sweep_row(const DevParams& P, const StateView&
             }
         } else {
             // scalar reconstructions: one component of the window at a time
-            auto P = [&](int m, int q) { return ring.comp(wq, cell[m], q, false); };
-            auto M = [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); };
+            auto plus = [&](int m, int q) { return ring.comp(wq, cell[m], q, false); };
+            auto minus = [&](int m, int q) { return ring.comp(wq, cell[S - 1 - m], q, true); };
             if constexpr (sizeof(R) == 8) {
                 recon_words<RC>([&](int m, int k) { return ring.a[wq][k][cell[m]]; }, lin, disp, diss, face);
-                recon_face_huge<R, RC, true>(P, M, face);
+                recon_face_huge<R, RC, true>(plus, minus, face);
             } else {
-                recon_face<R, RC, true>(P, M, lin, disp, diss, face);
+                recon_face<R, RC, true>(plus, minus, lin, disp, diss, face);
             }
         }
     };
@@ -1586,7 +1586,8 @@ __device__ __forceinline__ void stage_cell(const DevParams& P, const StateView& 
 // 8 blocks of 128 threads per SM (at most 64 registers): the neighbour loads
 // are latency-bound, and more resident warps beat more loads in flight per
 // thread. Measured at 256^3: FP32 0.713 -> 0.578 ms (5 blocks 0.630, 7 blocks
-// 0.609, 10 blocks 0.680); FP64 1.80 -> 1.39 ms (6 blocks 1.52, 10 blocks 1.55).
+// 0.609, 10 blocks 0.680); FP64 with the compiler's divisions 1.80 -> 1.39 ms (6
+// blocks 1.52, 10 blocks 1.55), with div_wide 1.02.
 template <class R, int ORD, int STAGE, bool T3 = false>
 __global__ void __launch_bounds__(128, 8)
 k_update(DevParams P, StateView Wc, StateView W0, const R* __restrict__ tacc,
@@ -1765,13 +1766,13 @@ k_sweep_ring(DevParams P, StateView W, R* __restrict__ tacc, int seg, const Ctrl
                 int sl[S];
 #pragma unroll
                 for (int m = 0; m < S; ++m) sl[m] = ph + m < S ? ph + m : ph + m - S;
-                auto P = [&](int m, int q) { return ring.comp(sl[m], tid, q, false); };
-                auto M = [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); };
+                auto plus = [&](int m, int q) { return ring.comp(sl[m], tid, q, false); };
+                auto minus = [&](int m, int q) { return ring.comp(sl[S - 1 - m], tid, q, true); };
                 if constexpr (sizeof(R) == 8) {
                     recon_words<RC>([&](int m, int k) { return ring.a[sl[m]][k][tid]; }, lin, disp, diss, face);
-                    recon_face_huge<R, RC, true>(P, M, face);
+                    recon_face_huge<R, RC, true>(plus, minus, face);
                 } else {
-                    recon_face<R, RC, true>(P, M, lin, disp, diss, face);
+                    recon_face<R, RC, true>(plus, minus, lin, disp, diss, face);
                 }
             }
             if (t > 0) {

@@ -92,13 +92,18 @@ inline int segment_for(int len, long long lines) {
 
 }  // namespace detail
 
-// Whether an FP64 box takes launch_flux_small: every line short enough for a block's shared memory, no tuning override of the
-// marching kernels, and few enough cells: L.small (1500000) where nx is a
-// multiple of 32 and the x sweep marches a warp per row (a step at 64^3 356 ->
-// 265 us, 112^3 1917 -> 1508 us WENO5 and 1214 -> 1044 us MDCD; 128^3 2092 -> 2102
-// and 1319 -> 1456), six times as many elsewhere, where it marches a thread per
-// row (100x75x90 1203 -> 773 us, 200^3 10.2 -> 8.6 ms WENO5, 6.6 -> 6.2 ms MDCD;
-// larger ones not measured).
+// Whether an FP64 box takes launch_flux_small: every line short enough for a
+// block's shared memory, no tuning override of the marching kernels, and few
+// enough cells: L.small (1500000) where nx is a multiple of 32 and the x sweep
+// marches a warp per row (a step at 64^3 356 -> 265 us, 112^3 1917 -> 1508 us
+// WENO5 and 1214 -> 1044 us MDCD; 128^3 2092 -> 2102 and 1319 -> 1456; flat boxes just
+// below the limit gain in WENO5, 32x216x216 1876 -> 1694, and lose in MDCD, 1182 -> 1323),
+// six times as many elsewhere, where it marches a thread per row (100x75x90 1203 ->
+// 773 us, 200^3 10.2 -> 8.6 ms WENO5, 6.6 -> 6.2 ms MDCD) and with characteristic-wise
+// reconstruction (200^3 16.2 -> 12.9 ms, 12.5 -> 11.0). With one line a block along y and
+// z: 30x390x390 6.25 -> 5.18 ms WENO5, 4.05 -> 4.06 MDCD; 300x300x90 10.0 -> 9.11, 6.62 ->
+// 6.73; 210x210x200 11.0 -> 9.68, 7.34 -> 7.36; characteristic 100x290x300 17.8 -> 13.6, 14.0 ->
+// 11.4, 160^3 8.41 -> 6.57, 6.32 -> 6.02. (Marching kernels -> k_flux_small throughout.)
 inline bool small_box(const LaunchCfg& L) {
     const DevParams& P = L.P;
     const int most = small_most(L.chr != 0);
@@ -120,6 +125,9 @@ inline bool small_box(const LaunchCfg& L) {
 // viscous terms or Lax-Friedrichs + WENO5 and all but the two-point scheme (LF MDCD
 // 54x43x47 185 -> 209, 53x26x54 166 -> 183, 49x37x46 180 -> 192, LF WENO5 55x54x46 213 -> 238;
 // smaller and larger ones gain, LF MDCD 34^3 153 -> 141, 52^3 207 -> 183).
+// Characteristic-wise and MDCD_HYBRID boxes above 30000 cells are left out on no
+// more than caution: overlapped they would gain on warp rows (64^3 FP64 369 -> 353 and
+// 383 -> 368 us, FP32 373 -> 336 and 327 -> 294; 80^3 FP64 equal; 40^3 FP32 equal).
 inline bool pdl_box(const LaunchCfg& L, bool fp64) {
     const DevParams& P = L.P;
     const long long n = P.n;
@@ -420,7 +428,8 @@ cudaError_t launch_rhs_out(const LaunchCfg& L, const R* tacc, const R* fv, doubl
 namespace detail {
 template <int FVS, int RC, bool CHR>
 cudaError_t flux_small(const LaunchCfg& L, StateView W, double* tacc, double* fv, const Ctrl* ctrl) {
-    // 64 to 256 cells a block, so that the three sweeps give at least two blocks per SM
+    // 64 to 256 cells a block: the three sweeps together give two blocks per SM or
+    // more from 6300 cells on (below, blocks of 64 cells are fewer)
     const long long target = std::min(256ll, std::max(64ll, 3 * L.P.n / (2 * 148)));
     const SmallShape sh = small_shape(L.P, target, small_most(CHR), SMALL_T);
     const int nc = small_cells(L.P, sh);

@@ -10,9 +10,9 @@
 // input and output buffers; the intermediate arrays of the RHS live in a
 // fixed-size array of this library's own device memory.
 //
-// The scratch (temperature + the inviscid accumulator + the viscous fluxes)
-// is the file-scope array below: 15 doubles per cell for at most
-// NS3D_NOALLOC_MAX_CELLS cells, 7.5 MiB, held on every GPU that loads the
+// The scratch (temperature + the inviscid accumulator or, up to 39321 cells of the
+// FP64 form, the three directions' terms + the viscous fluxes) is the file-scope array
+// below: 15 doubles for each of NS3D_NOALLOC_MAX_CELLS cells, 7.5 MiB, held on every GPU that loads the
 // library until the process exits. Every call shares it and it keeps the last
 // call's contents; each kernel overwrites what it reads later in the same
 // call, so nothing needs clearing, but calls that overlap on the GPU (other
@@ -37,8 +37,9 @@ extern template cudaError_t launch_visc_flux<float>(const LaunchCfg&, StateView,
 extern template cudaError_t launch_rhs_out<float>(const LaunchCfg&, const float*, const float*, double*);
 }  // namespace ns3d
 
-// 15 doubles per cell: T (double) + 5 accumulator values + the viscous fluxes
-// (9 doubles in the FP64 form; 5 + 12 floats in the FP32-stencil form).
+// Per cell: T (double) + 5 accumulator values + the viscous fluxes (9 doubles in
+// the FP64 form, 15 in all; 5 + 12 floats in the FP32-stencil form), or the FP64 form's
+// separate terms, 1 + 15 + 9 doubles, where 25 a cell fit the whole array (rhs_into).
 static __device__ __align__(256) double g_noalloc_scratch[15 * (long long)NS3D_NOALLOC_MAX_CELLS];
 
 namespace {

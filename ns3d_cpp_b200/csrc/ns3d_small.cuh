@@ -32,8 +32,10 @@ struct SmallShape {
     int nb[4], lb[3];
 };
 
-// `target` cells per block (lines of up to `most` cells), four lines or more
-// along y and z (32-byte rows); `vth` cells per block of the fourth role.
+// `target` cells per block, four lines or more along y and z (32-byte rows) as
+// far as `most` cells hold them: with 400 (300) extents above 100 (75) have three
+// lines, above 200 (150) one, whose loads and stores use 8 bytes of a sector. That still beats
+// the marching kernels (see small_box). `vth`: cells per block of the fourth role.
 inline SmallShape small_shape(const DevParams& P, long long target, int most, int vth) {
     SmallShape sh{};
     for (int d = 0; d < 3; ++d) {
@@ -351,8 +353,10 @@ k_flux_small(DevParams P, StateView W, double* __restrict__ t3, double* __restri
 // the fifth the two conserved states, then the stage: a quarter of k_update's 96
 // neighbour loads per thread one after the other, which is what bounds it there
 // (a stage at 16^3: 6 us against 8; from 48^3 on k_update's larger number of
-// cells in flight is the better one; four warps, with the stage in warp 0,
-// measured 2% slower than five).
+// cells in flight is the better one; between 32^3 and 48^3 not measured; four warps,
+// with the stage in warp 0, measured 2% slower than five). STAGE 0 has no wider
+// form: a right-hand side's kernels, marching ones with k_rhs_out -> k_flux_small with
+// this: 48^3 136 -> 57 us, 100^3 534 -> 392 us, 200^3 3.21 -> 2.96 ms.
 template <int ORD, int STAGE>
 __global__ void __launch_bounds__(160)
 k_update_small(DevParams P, StateView Wc, StateView W0, const double* __restrict__ t3,
