@@ -1487,8 +1487,17 @@ ns3d_status ns3d_energy_spectrum(ns3d_ctx* ctx, double* Ek, int nbins) {
     NS3D_CK(cudaMemsetAsync(ctx->bins, 0, sizeof(double) * kmax, ctx->stream));
     const double scale = 1.0 / (double)ctx->n;  // EnergySpectrum.cpp:88-96
     const int nbu = spectrum_bins_used(nx, ny, nz);
+    const int tmpb = ctx->cur == ctx->rec ? (ctx->cur + 1) % 3 : 3 - ctx->cur - ctx->rec;
     for (int comp = 1; comp <= 3; ++comp) {
-        if (cufftExecD2Z(ctx->fft, warr(ctx, ctx->cur, comp), ctx->spec) != CUFFT_SUCCESS)
+        // cuFFT wants its input on a 16-byte boundary; with an odd number of cells u and
+        // w are not, and go through the first array of the free state buffer
+        double* in = warr(ctx, ctx->cur, comp);
+        if (reinterpret_cast<uintptr_t>(in) % 16 != 0) {
+            double* aligned = warr(ctx, tmpb, 0);
+            NS3D_CK(cudaMemcpyAsync(aligned, in, sizeof(double) * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
+            in = aligned;
+        }
+        if (cufftExecD2Z(ctx->fft, in, ctx->spec) != CUFFT_SUCCESS)
             return fail(ctx, NS3D_ERR_CUDA, "cufftExecD2Z failed");
         NS3D_LAUNCH(NS3D_KERNEL_OTHER, 2,
                     (k_spectrum_part<<<SPEC_BLOCKS, 32 * SPEC_WARPS,

@@ -118,3 +118,18 @@ def test_workload_reports_the_one_launch_fluxes():
     k = workloads.run_one(w, workloads.initial_for(w), "weno5", "fp64", 4, 0)["kernels"]
     assert k["fluxes"]["launches"] == k["update"]["launches"] == 12 and k["fluxes"]["hbm_frac"] > 0
     assert "sweep_x" not in k and "other" not in k
+
+
+@pytest.mark.parametrize("box", [(9, 11, 13), (15, 15, 15), (9, 11, 14)], ids=lambda b: "x".join(map(str, b)))
+def test_spectrum_of_an_odd_number_of_cells(oracle_mod, box):
+    """u and w of such a box start on an 8-byte boundary, which cuFFT refuses; the
+    spectrum and the state after it are as for any other box."""
+    W = _field(box)
+    with _solver(_box_params(box), {}) as s:
+        s.upload_primitive(W)
+        s.step(1)
+        res, state = s.residuals(), s.download_primitive()
+        E = s.compute_energy_spectrum()
+        assert np.array_equal(s.residuals(), res) and np.array_equal(s.download_primitive(), state)
+    want = oracle_mod.spectrum(*state[1:4])
+    assert E.shape == want.shape and np.all(np.abs(E - want) <= 1e-12 * want.max())
